@@ -90,8 +90,11 @@ typedef struct { zt_shape shape; zt_vec3 radiance; double weight; } zt_light;
 enum { ZT_MODE_AUTO = 0, ZT_MODE_MEGAKERNEL = 1, ZT_MODE_WAVEFRONT = 2, ZT_MODE_MEGAKERNEL_REGEN = 3,
        ZT_MODE_WAVEFRONT_SORTED = 4 };
 /* ZT_PRECISION_EXACT (the default) is the verification build of the path:
- * every operation is the reference's f64 operation in the reference's order,
- * so images are bit-identical to the reference algorithm's as restated by
+ * every value is the reference's f64 value, computed in the reference's
+ * order (BVH boxes of scenes with 64 or more bounded primitives are tested in
+ * single precision first, and every hit so found is checked to be the one the
+ * f64 walk finds; pixels where that is in doubt take the f64 walk), so images
+ * are bit-identical to the reference algorithm's as restated by
  * the project's CPU oracle (which shares this library's sin/cos, so parity
  * with Zig's own transcendentals is not covered).
  * ZT_PRECISION_FAST tests BVH boxes in single precision against conservative

@@ -293,22 +293,25 @@ static RenderParams make_params(const zt_scene* s, const zt_options* o) {
 /* ------------------------------------------------------------ Kernels ---- */
 
 /* One pixel: renderTile's per-pixel body, render.zig:133-144.  kNee as for
- * trace_with. */
-template <bool kAux, bool kNee = true, bool kFast = false>
-__device__ __forceinline__ void render_pixel(const DevScene& sc, const RenderParams& p, uint64_t pix,
+ * trace_with.  Returns false when the float walk could not be shown to give
+ * the f64 walk's paths; nothing is written then. */
+template <bool kAux, bool kNee, int kWalk>
+__device__ __forceinline__ bool render_pixel(const DevScene& sc, const RenderParams& p, uint64_t pix,
                                              double* __restrict__ out, TraceAux* aux) {
   const uint64_t x = pix % p.width, y = pix / p.width;
   const double w = (double)p.width, h = (double)p.height;
   const double inv_spp = 1.0 / (double)p.spp;
   Rng rng = rng_for_stream(p.seed, y * p.width + x);
   dv3 sum = V(0, 0, 0);
+  bool unsure = false;
   for (uint64_t i = 0; i < p.spp; ++i) {
     const double s = ((double)x + rng_float(rng)) / w;
     const double t = ((double)y + rng_float(rng)) / h;
     dv3 ro, rd;
     camera_ray(p.cam, s, t, rng, ro, rd);
-    const dv3 c = trace_with<kAux, kNee, kFast>(sc, ro, rd, rng, p.max_depth, p.use_nee != 0, aux);
+    const dv3 c = trace_with<kAux, kNee, kWalk>(sc, ro, rd, rng, p.max_depth, p.use_nee != 0, aux, unsure);
     if (kAux) break;
+    if (kWalk != kWalkF64 && unsure) return false;
     if (visfinite(c)) sum = sum + c;
   }
   if (!kAux) {
@@ -318,17 +321,26 @@ __device__ __forceinline__ void render_pixel(const DevScene& sc, const RenderPar
     out[3 * o + 1] = px.y;
     out[3 * o + 2] = px.z;
   }
+  return true;
+}
+
+/* The pixel with the f64 walk, called where the float walk was unsure. */
+__device__ __noinline__ void render_pixel_f64(const DevScene& sc, const RenderParams& p, uint64_t pix,
+                                              double* __restrict__ out) {
+  render_pixel<false, true, kWalkF64>(sc, p, pix, out, nullptr);
 }
 
 /* Persistent megakernel: each warp takes an 8x4 pixel tile from the device
  * work counter until the image is exhausted (the device form of
  * Context.work's atomic tile counter, render.zig:113-119), so its camera rays
- * are coherent.  The exact instance with light sampling is built for 1024
+ * are coherent.  The f64-walk instance with light sampling is built for 1024
  * resident threads per SM (64 registers): on the 1M-triangle terrain 731
  * Msamples/s against 722 at 896 (an earlier source measured 896 fastest).
- * The instance without light sampling (kNee = false) is a separate build
- * with its own residency: 896 threads (72 registers), equal to 1024 on the
- * random spheres (2798 against 2794). */
+ * The f64-walk instance without light sampling (kNee = false) is a separate
+ * build with its own residency: 896 threads (72 registers), equal to 1024 on
+ * the random spheres (2798 against 2794).
+ * The scene and parameters are __grid_constant__: render_pixel_f64 takes them
+ * by reference, and without it every thread would copy them to its stack. */
 constexpr int kMegaThreadsPerSm = 1024;
 constexpr int kMegaThreadsPerSmNoNee = 896;
 #ifndef ZT_FAST_THREADS_PER_SM
@@ -342,14 +354,14 @@ constexpr int kMegaThreadsPerSmNoNee = 896;
  * fast-walk instances measured fastest at 1024 (64 registers): on the
  * 1M-triangle terrain 1026 Msamples/s against 992 at 896 and 933 at 768; on
  * the sphere-field batch 64.4 ms against 67.9 at 896 and 71.7 at 1280. */
-__host__ __device__ constexpr int mega_threads_per_sm(bool nee, bool fast) {
-  return fast ? (nee ? ZT_FAST_THREADS_PER_SM : ZT_FAST_THREADS_PER_SM_NONEE)
-              : (nee ? kMegaThreadsPerSm : kMegaThreadsPerSmNoNee);
+__host__ __device__ constexpr int mega_threads_per_sm(bool nee, int walk) {
+  return walk != kWalkF64 ? (nee ? ZT_FAST_THREADS_PER_SM : ZT_FAST_THREADS_PER_SM_NONEE)
+                          : (nee ? kMegaThreadsPerSm : kMegaThreadsPerSmNoNee);
 }
 
-template <int BS, bool kNee, bool kFast = false>
-__global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kFast) / BS)
-    k_render_mega(DevScene sc, RenderParams p, double* __restrict__ out, unsigned int* __restrict__ counter) {
+template <int BS, bool kNee, int kWalk>
+__global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kWalk) / BS)
+    k_render_mega(const __grid_constant__ DevScene sc, const __grid_constant__ RenderParams p, double* __restrict__ out, unsigned int* __restrict__ counter) {
   const uint64_t tiles_x = (p.width + 7) / 8, tiles = tiles_x * ((p.rows + 3) / 4);
   const uint64_t row_end = p.row0 + p.rows;
   const unsigned lane = threadIdx.x & 31;
@@ -359,7 +371,8 @@ __global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kFast) / BS)
     tile = __shfl_sync(0xffffffffu, tile, 0);
     if ((uint64_t)tile >= tiles) return;
     const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    if (x < p.width && y < row_end) render_pixel<false, kNee, kFast>(sc, p, y * p.width + x, out, nullptr);
+    if (x < p.width && y < row_end && !render_pixel<false, kNee, kWalk>(sc, p, y * p.width + x, out, nullptr))
+      render_pixel_f64(sc, p, y * p.width + x, out);
   }
 }
 
@@ -372,7 +385,7 @@ __global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kFast) / BS)
  * valid = false).  Pays off when path lengths vary widely within a warp
  * (closed scenes such as the Cornell box); on open scenes with short paths
  * the nested form is faster. */
-template <bool kFast>
+template <int kWalk>
 __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const RenderParams& p, uint64_t x, uint64_t y,
                                                    bool valid, double* __restrict__ out) {
   const double w = (double)p.width, h = (double)p.height;
@@ -380,7 +393,7 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
   Rng rng = rng_for_stream(p.seed, valid ? y * p.width + x : 0);
   dv3 sum = V(0, 0, 0);
   uint64_t sample = 0, depth = 0;
-  bool done = !valid, fresh = valid;
+  bool done = !valid, fresh = valid, unsure = false;
   /* prev_origin (render.zig:66-70) is read only after a bounce, where it
    * equals ro: ro stands in for it, as in trace_with */
   dv3 ro = V(0, 0, 0), rd = V(0, 0, 0), radiance = V(0, 0, 0), throughput = V(1, 1, 1);
@@ -406,18 +419,18 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
     bool end = depth >= p.max_depth;
     if (!end) {
       Hit hit;
-      if (!scene_intersect<false, kFast>(sc, ro, rd, kRayEpsilon, INFINITY, hit)) {
+      if (!scene_intersect<kWalk>(sc, ro, rd, kRayEpsilon, INFINITY, hit, unsure)) {
         radiance = radiance + vmul(throughput, background_radiance(sc.bg, rd));
         end = true;
       } else {
         const DMat& mat = sc.mats[hit.material];
         const dv3 le = (mat.kind == kEmissive && hit.front_face) ? L3(mat.color) : V(0, 0, 0);
         if (vmaxc(le) > 0) {
-          const double wt = prev_pdf > 0 ? power_weight(prev_pdf, lights_pdf_hit<kFast>(sc, ro, hit.point)) : 1.0;
+          const double wt = prev_pdf > 0 ? power_weight(prev_pdf, lights_pdf_hit<kWalk != kWalkF64>(sc, ro, hit.point)) : 1.0;
           radiance = radiance + vscale(vmul(throughput, le), wt);
         }
         if (mat.kind == kLambertian && use_nee)
-          radiance = radiance + vmul(throughput, direct_light<kFast>(sc, L3(mat.color), hit, rng));
+          radiance = radiance + vmul(throughput, direct_light<kWalk>(sc, L3(mat.color), hit, rng, unsure));
         dv3 atten, sd;
         if (!material_scatter(mat, rd, hit, rng, atten, sd)) {
           end = true;
@@ -440,9 +453,12 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
       if (visfinite(radiance)) sum = sum + radiance;
       ++sample;
       fresh = true;
+      if (kWalk != kWalkF64 && unsure) sample = p.spp; /* give the pixel up: rendered again below */
     }
   }
-  if (valid) {
+  if (kWalk != kWalkF64 && unsure) {
+    render_pixel_f64(sc, p, y * p.width + x, out);
+  } else if (valid) {
     const dv3 px = vscale(sum, 1.0 / (double)p.spp);
     const uint64_t o = (y - p.row0) * p.width + x;
     out[3 * o + 0] = px.x;
@@ -455,8 +471,9 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
  * per SM (up to 128 registers, no spills): 1.17x the seven-block build on the
  * Cornell box, whose 65,536 pixels fill only a quarter of the GPU's thread
  * slots anyway, and equal to it on 1280x720 random spheres. */
-template <int BS, bool kFast = false>
-__global__ void __launch_bounds__(BS, 512 / BS) k_render_regen(DevScene sc, RenderParams p, double* __restrict__ out,
+template <int BS, int kWalk>
+__global__ void __launch_bounds__(BS, 512 / BS) k_render_regen(const __grid_constant__ DevScene sc,
+                                                             const __grid_constant__ RenderParams p, double* __restrict__ out,
                                                              unsigned int* __restrict__ counter) {
   const uint64_t tiles_x = (p.width + 7) / 8, tiles = tiles_x * ((p.rows + 3) / 4);
   const uint64_t row_end = p.row0 + p.rows;
@@ -467,7 +484,7 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_render_regen(DevScene sc, Rend
     tile = __shfl_sync(0xffffffffu, tile, 0);
     if ((uint64_t)tile >= tiles) return;
     const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    render_pixel_regen<kFast>(sc, p, x, y, x < p.width && y < row_end, out);
+    render_pixel_regen<kWalk>(sc, p, x, y, x < p.width && y < row_end, out);
   }
 }
 
@@ -487,8 +504,8 @@ struct BatchItem {
  * render them with the item's own scene and parameters, so small images do
  * not leave the GPU idle the way one launch per image does.  kNee = false
  * is the instance for batches in which no render samples lights. */
-template <int BS, bool kNee, bool kFast = false>
-__global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kFast) / BS)
+template <int BS, bool kNee, int kWalk>
+__global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kWalk) / BS)
     k_render_batch(const BatchItem* __restrict__ items, uint32_t n_items, uint64_t total_tiles,
                    unsigned int* __restrict__ counter) {
   const unsigned lane = threadIdx.x & 31;
@@ -506,8 +523,9 @@ __global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kFast) / BS)
     const BatchItem& it = items[lo];
     const uint64_t local = tile - it.tile_begin;
     const uint64_t x = (local % it.tiles_x) * 8 + (lane & 7), y = (local / it.tiles_x) * 4 + (lane >> 3);
-    if (x < it.p.width && y < it.p.height)
-      render_pixel<false, kNee, kFast>(it.sc, it.p, y * it.p.width + x, it.out, nullptr);
+    if (x < it.p.width && y < it.p.height &&
+        !render_pixel<false, kNee, kWalk>(it.sc, it.p, y * it.p.width + x, it.out, nullptr))
+      render_pixel_f64(it.sc, it.p, y * it.p.width + x, it.out);
   }
 }
 
@@ -516,7 +534,7 @@ __global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kFast) / BS)
  * next sample at once.  Built like k_render_regen (four blocks of 128 per
  * SM, 128 registers).  Every lane of a warp calls render_pixel_regen, lanes
  * outside their image with valid = false. */
-template <int BS, bool kFast>
+template <int BS, int kWalk>
 __global__ void __launch_bounds__(BS, 512 / BS)
     k_render_batch_regen(const BatchItem* __restrict__ items, uint32_t n_items, uint64_t total_tiles,
                          unsigned int* __restrict__ counter) {
@@ -535,7 +553,7 @@ __global__ void __launch_bounds__(BS, 512 / BS)
     const BatchItem& it = items[lo];
     const uint64_t local = tile - it.tile_begin;
     const uint64_t x = (local % it.tiles_x) * 8 + (lane & 7), y = (local / it.tiles_x) * 4 + (lane >> 3);
-    render_pixel_regen<kFast>(it.sc, it.p, x, y, x < it.p.width && y < it.p.height, it.out);
+    render_pixel_regen<kWalk>(it.sc, it.p, x, y, x < it.p.width && y < it.p.height, it.out);
   }
 }
 
@@ -544,7 +562,7 @@ __global__ void k_render_debug(DevScene sc, RenderParams p, int32_t* __restrict_
   const uint64_t pix = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (pix >= p.width * p.height) return;
   TraceAux aux;
-  render_pixel<true>(sc, p, pix, nullptr, &aux);
+  render_pixel<true, true, kWalkF64>(sc, p, pix, nullptr, &aux);
   first_prim[pix] = aux.first_prim;
   path_len[pix] = aux.path_len;
 }
@@ -843,7 +861,8 @@ __global__ void k_trace_paths(DevScene sc, double ox, double oy, double oz, doub
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   Rng rng{rng_state[0], rng_state[1], rng_state[2], rng_state[3]};
   for (uint64_t i = 0; i < n; ++i) {
-    const dv3 c = trace_with<false>(sc, V(ox, oy, oz), V(dx, dy, dz), rng, max_depth, use_nee != 0, nullptr);
+    bool unsure = false;
+    const dv3 c = trace_with<false, true, kWalkF64>(sc, V(ox, oy, oz), V(dx, dy, dz), rng, max_depth, use_nee != 0, nullptr, unsure);
     out[3 * i + 0] = c.x;
     out[3 * i + 1] = c.y;
     out[3 * i + 2] = c.z;
@@ -882,57 +901,61 @@ static unsigned persistent_grid(K kernel, int block, uint64_t work_items, size_t
 enum MegaVariant { kMegaNested = 0, kMegaRegen = 1 };
 constexpr double kRegenMeanPath = 3.0;
 
-template <int BS, bool kFast>
+template <int BS, int kWalk>
 static void launch_mega_bsf(const DevScene& v, const RenderParams& p, double* d_out, unsigned int* counter,
                             MegaVariant variant, cudaStream_t stream) {
   const uint64_t npix = p.width * p.rows;
   if (variant == kMegaRegen)
-    k_render_regen<BS, kFast><<<persistent_grid(k_render_regen<BS, kFast>, BS, npix), BS, 0, stream>>>(v, p, d_out,
+    k_render_regen<BS, kWalk><<<persistent_grid(k_render_regen<BS, kWalk>, BS, npix), BS, 0, stream>>>(v, p, d_out,
                                                                                                       counter);
   else if (p.use_nee)
-    k_render_mega<BS, true, kFast><<<persistent_grid(k_render_mega<BS, true, kFast>, BS, npix), BS, 0, stream>>>(
+    k_render_mega<BS, true, kWalk><<<persistent_grid(k_render_mega<BS, true, kWalk>, BS, npix), BS, 0, stream>>>(
         v, p, d_out, counter);
   else
-    k_render_mega<BS, false, kFast><<<persistent_grid(k_render_mega<BS, false, kFast>, BS, npix), BS, 0, stream>>>(
+    k_render_mega<BS, false, kWalk><<<persistent_grid(k_render_mega<BS, false, kWalk>, BS, npix), BS, 0, stream>>>(
         v, p, d_out, counter);
 }
 
 template <int BS>
 static void launch_mega_bs(const DevScene& v, const RenderParams& p, double* d_out, unsigned int* counter,
-                           MegaVariant variant, bool fast, cudaStream_t stream) {
-  if (fast) launch_mega_bsf<BS, true>(v, p, d_out, counter, variant, stream);
-  else launch_mega_bsf<BS, false>(v, p, d_out, counter, variant, stream);
+                           MegaVariant variant, Walk walk, cudaStream_t stream) {
+  if (walk == kWalkFloat) launch_mega_bsf<BS, kWalkFloat>(v, p, d_out, counter, variant, stream);
+  else if (walk == kWalkFloatChecked) launch_mega_bsf<BS, kWalkFloatChecked>(v, p, d_out, counter, variant, stream);
+  else launch_mega_bsf<BS, kWalkF64>(v, p, d_out, counter, variant, stream);
 }
 
 static bool valid_block_size(uint32_t bs) { return bs == 0 || bs == 64 || bs == 128 || bs == 256; }
 
-/* Whether a render takes the fast traversal: asked for, the scene has its
- * float records (a scene whose leaves or bounds do not fit them renders
- * with the f64 traversal) and, for a single render, at least
- * kFastMinPrimitives bounded primitives.  The camera origin must be within
- * the records' coordinate range as well. */
+/* The walk a render takes.  The float walk needs the scene's float records
+ * and a camera origin within their coordinate range; ZT_PRECISION_EXACT also
+ * needs boxes that its hits can be checked against (verify_ok) and walks
+ * checked.  A single render needs at least kFastMinPrimitives bounded
+ * primitives: on a tree this small the float walk's per-ray set-up costs more
+ * than its box tests save (Cornell box, 14 primitives: 477 against 565
+ * Msamples/s); a batch, whose renders share one kernel instance, skips this
+ * rule. */
 constexpr uint32_t kFastMinPrimitives = 64;
-static bool use_fast(const zt_scene* s, const RenderParams& p, uint32_t precision, bool small_scenes_exact = true) {
-  if (precision != ZT_PRECISION_FAST || !s->device || !s->device->view.fast_ok) return false;
-  /* on a tree this small the float walk's per-ray set-up costs more than its
-   * box tests save (Cornell box, 14 primitives: 477 vs 565 Msamples/s); a
-   * batch, whose renders share one kernel instance, skips this rule */
-  if (small_scenes_exact && s->device->view.n_prims < kFastMinPrimitives) return false;
+static Walk choose_walk(const zt_scene* s, const RenderParams& p, uint32_t precision, bool small_scenes_f64 = true) {
+  if (!s->device || !s->device->view.fast_ok) return kWalkF64;
+  if (precision != ZT_PRECISION_FAST && !s->device->view.verify_ok) return kWalkF64;
+  if (small_scenes_f64 && s->device->view.n_prims < kFastMinPrimitives) return kWalkF64;
   const double* o = p.cam.origin;
   const double reach = fabs(p.cam.lens_radius) * (fabs(p.cam.u[0]) + fabs(p.cam.u[1]) + fabs(p.cam.u[2]) +
                                                   fabs(p.cam.v[0]) + fabs(p.cam.v[1]) + fabs(p.cam.v[2]));
-  return fabs(o[0]) + reach <= kFastMaxCoord && fabs(o[1]) + reach <= kFastMaxCoord &&
-         fabs(o[2]) + reach <= kFastMaxCoord;
+  const bool near = fabs(o[0]) + reach <= kFastMaxCoord && fabs(o[1]) + reach <= kFastMaxCoord &&
+                    fabs(o[2]) + reach <= kFastMaxCoord;
+  if (!near) return kWalkF64;
+  return precision == ZT_PRECISION_FAST ? kWalkFloat : kWalkFloatChecked;
 }
 
 static zt_status launch_mega(zt_scene* s, const RenderParams& p, uint32_t block_size, double* d_out,
-                             MegaVariant variant, bool fast, cudaStream_t stream) {
+                             MegaVariant variant, Walk walk, cudaStream_t stream) {
   zt_device_buffers* d = s->device;
   ZT_CUDA(cudaMemsetAsync(d->counter, 0, sizeof(unsigned int), stream), "reset work counter");
   const DevScene v = launch_view(s);
-  if (block_size == 64) launch_mega_bs<64>(v, p, d_out, d->counter, variant, fast, stream);
-  else if (block_size == 256) launch_mega_bs<256>(v, p, d_out, d->counter, variant, fast, stream);
-  else launch_mega_bs<128>(v, p, d_out, d->counter, variant, fast, stream);
+  if (block_size == 64) launch_mega_bs<64>(v, p, d_out, d->counter, variant, walk, stream);
+  else if (block_size == 256) launch_mega_bs<256>(v, p, d_out, d->counter, variant, walk, stream);
+  else launch_mega_bs<128>(v, p, d_out, d->counter, variant, walk, stream);
   ZT_CUDA(cudaGetLastError(), "launch the megakernel");
   return ZT_OK;
 }
@@ -1123,7 +1146,7 @@ static zt_status launch_render_params(zt_scene* s, const RenderParams& p, const 
   const bool long_paths = s->pilot_valid && s->mean_path >= kRegenMeanPath;
   const MegaVariant variant =
       (mode == ZT_MODE_MEGAKERNEL_REGEN || (mode == ZT_MODE_AUTO && long_paths)) ? kMegaRegen : kMegaNested;
-  return launch_mega(s, p, bs, d_out, variant, use_fast(s, p, precision), stream);
+  return launch_mega(s, p, bs, d_out, variant, choose_walk(s, p, precision), stream);
 }
 
 static zt_status launch_render(zt_scene* s, const zt_options* o, const zt_gpu_config* cfg, double* d_out,
@@ -1300,7 +1323,7 @@ zt_status zt_render_rows(zt_scene* s, const zt_options* o, uint64_t row_begin, u
   double* d_out = nullptr;
   if ((rc = pool_alloc((void**)&d_out, bytes, 0, "allocate framebuffer band")) != ZT_OK) return rc;
   rc = launch_mega(s, p, 0, d_out, s->pilot_valid && s->mean_path >= kRegenMeanPath ? kMegaRegen : kMegaNested,
-                   false, 0);
+                   choose_walk(s, p, ZT_PRECISION_EXACT), 0);
   if (rc == ZT_OK) {
     cudaError_t e = cudaMemcpyAsync(out, d_out, bytes, cudaMemcpyDeviceToHost, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
@@ -1739,7 +1762,7 @@ struct zt_batch {
   uint64_t total_tiles = 0;
   uint32_t block_size = 128;
   bool nee = true; /* some render of the batch samples lights */
-  bool fast = false; /* every render takes the fast traversal */
+  Walk walk = kWalkF64; /* the float walk only if every render can take it */
   bool regen = false; /* the path-regeneration form of the batched kernel */
   BatchItem* d_items = nullptr;
   unsigned int* d_counter = nullptr;
@@ -1748,34 +1771,32 @@ struct zt_batch {
 
 namespace zt {
 
-template <int BS, bool kNee, bool kFast>
+template <int BS, bool kNee, int kWalk>
 static void launch_batch_kernel(const zt_batch* b, cudaStream_t st) {
-  k_render_batch<BS, kNee, kFast>
-      <<<persistent_grid(k_render_batch<BS, kNee, kFast>, BS, b->total_tiles * 32), BS, 0, st>>>(
+  k_render_batch<BS, kNee, kWalk>
+      <<<persistent_grid(k_render_batch<BS, kNee, kWalk>, BS, b->total_tiles * 32), BS, 0, st>>>(
           b->d_items, (uint32_t)b->n, b->total_tiles, b->d_counter);
 }
 
-template <int BS, bool kFast>
+template <int BS, int kWalk>
 static void launch_batch_regen(const zt_batch* b, cudaStream_t st) {
-  k_render_batch_regen<BS, kFast>
-      <<<persistent_grid(k_render_batch_regen<BS, kFast>, BS, b->total_tiles * 32), BS, 0, st>>>(
+  k_render_batch_regen<BS, kWalk>
+      <<<persistent_grid(k_render_batch_regen<BS, kWalk>, BS, b->total_tiles * 32), BS, 0, st>>>(
           b->d_items, (uint32_t)b->n, b->total_tiles, b->d_counter);
+}
+
+template <int BS, int kWalk>
+static void launch_batch_walk(const zt_batch* b, cudaStream_t st) {
+  if (b->regen) launch_batch_regen<BS, kWalk>(b, st);
+  else if (b->nee) launch_batch_kernel<BS, true, kWalk>(b, st);
+  else launch_batch_kernel<BS, false, kWalk>(b, st);
 }
 
 template <int BS>
 static void launch_batch_bs(const zt_batch* b, cudaStream_t st) {
-  if (b->regen) {
-    if (b->fast) launch_batch_regen<BS, true>(b, st);
-    else launch_batch_regen<BS, false>(b, st);
-    return;
-  }
-  if (b->fast) {
-    if (b->nee) launch_batch_kernel<BS, true, true>(b, st);
-    else launch_batch_kernel<BS, false, true>(b, st);
-  } else {
-    if (b->nee) launch_batch_kernel<BS, true, false>(b, st);
-    else launch_batch_kernel<BS, false, false>(b, st);
-  }
+  if (b->walk == kWalkFloat) launch_batch_walk<BS, kWalkFloat>(b, st);
+  else if (b->walk == kWalkFloatChecked) launch_batch_walk<BS, kWalkFloatChecked>(b, st);
+  else launch_batch_walk<BS, kWalkF64>(b, st);
 }
 
 static void batch_free(zt_batch* b) {
@@ -1845,9 +1866,10 @@ zt_status zt_batch_create(zt_scene* const* scenes, const zt_options* opts, uint6
     delete b;
     return fail(ZT_ERR_INVALID_ARGUMENT, "unknown zt_gpu_config.precision");
   }
-  b->fast = precision == ZT_PRECISION_FAST;
   b->regen = bmode == ZT_MODE_MEGAKERNEL_REGEN;
-  for (uint64_t k = 0; k < n && b->fast; ++k) b->fast = use_fast(scenes[idx[k]], items[k].p, precision, false);
+  b->walk = choose_walk(scenes[idx[0]], items[0].p, precision, false);
+  for (uint64_t k = 1; k < n && b->walk != kWalkF64; ++k)
+    b->walk = choose_walk(scenes[idx[k]], items[k].p, precision, false);
   cudaError_t e = cudaGetDevice(&b->device);
   if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_items, n * sizeof(BatchItem));
   if (e == cudaSuccess) e = cudaMalloc((void**)&b->d_counter, sizeof(unsigned int));
@@ -1950,7 +1972,7 @@ __global__ void __launch_bounds__(128, 7) k_render_mega_noalloc(DevScene sc, Ren
     tile = __shfl_sync(0xffffffffu, tile, 0);
     if ((uint64_t)tile >= tiles) return;
     const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = (tile / tiles_x) * 4 + (lane >> 3);
-    if (x < p.width && y < p.height) render_pixel<false>(sc, p, y * p.width + x, out, nullptr);
+    if (x < p.width && y < p.height) render_pixel<false, true, kWalkF64>(sc, p, y * p.width + x, out, nullptr);
   }
 }
 

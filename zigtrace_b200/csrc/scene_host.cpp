@@ -279,12 +279,35 @@ zt_status build_scene(zt_scene* s, bool device, bool* used_device, double* build
       if (rc == ZT_OK && used_device) *used_device = true;
     }
     if (rc == ZT_DEVICE_BUILD_FALLBACK) rc = build_bvh(s);
+    s->boxes_nested = true;
     if (rc == ZT_OK) rc = build_lights(s);
   } catch (const std::bad_alloc&) {
     return fail(ZT_ERR_OUT_OF_MEMORY, "OutOfMemory during Scene.build");
   }
   if (rc == ZT_OK) s->built = true;
   return rc;
+}
+
+/* Whether every node's box holds its children's boxes and, for a leaf, its
+ * primitives' (true of every tree Bvh.build makes, up to the sign of zero). */
+static bool boxes_nested(const zt_scene* s) {
+  auto holds = [](const HostNode& n, const double mn[3], const double mx[3]) {
+    for (int k = 0; k < 3; ++k)
+      if (!(n.bmin[k] <= mn[k] && mx[k] <= n.bmax[k])) return false;
+    return true;
+  };
+  for (const HostNode& n : s->nodes) {
+    if (n.count == 0) {
+      for (uint32_t c = n.first; c <= n.first + 1; ++c)
+        if (!holds(n, s->nodes[c].bmin, s->nodes[c].bmax)) return false;
+      continue;
+    }
+    for (uint32_t k = n.first; k < n.first + n.count; ++k) {
+      Box b = box_empty();
+      if (!shape_bounds(s->shapes[s->indices[k]], b) || !holds(n, b.mn, b.mx)) return false;
+    }
+  }
+  return true;
 }
 
 /* Scene.build with a BVH built elsewhere (the reference's own Bvh.build,
@@ -360,6 +383,7 @@ zt_status import_bvh(zt_scene* s, const zt_bvh_node* nodes, size_t n_nodes, cons
       h.count = nodes[i].count;
     }
     s->indices.assign(indices, indices + n);
+    s->boxes_nested = boxes_nested(s);
     const zt_status rc = build_lights(s);
     if (rc != ZT_OK) return rc;
   } catch (const std::bad_alloc&) {
@@ -492,6 +516,20 @@ static void make_fast_records(const zt_scene* s, FlatScene* f) {
   }
   v.froot_word = word(0);
   v.fast_ok = 1;
+  double reach = 0;
+  for (int k = 0; k < 3; ++k)
+    reach = std::max(reach, std::max(std::fabs(s->nodes[0].bmin[k]), std::fabs(s->nodes[0].bmax[k])));
+  v.freach = f32_up(reach);
+  /* walk_reaches (zt_fast.cuh) derives a leaf's box from its primitive: the
+   * tree's boxes must hold their contents, and no coordinate may be NaN
+   * (an infinite one exceeds kFastMaxCoord above) */
+  bool nan = false;
+  for (const DPrim& p : f->prims) {
+    double sum = 0;
+    for (int k = 0; k < 9; ++k) sum += p.a[k];
+    nan |= sum != sum;
+  }
+  v.verify_ok = s->boxes_nested && !nan;
 }
 
 void flatten_scene(const zt_scene* s, FlatScene* f) {

@@ -52,6 +52,7 @@ struct zt_scene {
   bool built = false;
   std::vector<zt::HostNode> nodes;
   std::vector<uint32_t> indices;
+  bool boxes_nested = false;  /* every node's box holds its children's and its primitives' boxes */
   std::vector<zt::HostLight> lights;
   std::vector<double> cdf;
   double total = 0;

@@ -133,6 +133,7 @@ ZT_D void hit_make(dv3 o, dv3 d, double t, dv3 outward, uint32_t mat, Hit& h) {
 
 /* Sphere.intersect, geometry.zig:37-52.  Returns the root t or a value
  * outside the range; the hit record is built only for the closest hit. */
+template <bool kInclusive = false>
 ZT_D bool sphere_t(dv3 center, double radius, dv3 o, dv3 d, double tmin, double tmax, double& tout) {
   const dv3 oc = center - o;
   const double a = vlen2(d);
@@ -142,9 +143,9 @@ ZT_D bool sphere_t(dv3 center, double radius, dv3 o, dv3 d, double tmin, double 
   if (disc < 0) return false;
   const double sq = sqrt(disc);
   double t = (h - sq) / a;
-  if (t <= tmin || t >= tmax) {
+  if (t <= tmin || (kInclusive ? t > tmax : t >= tmax)) {
     t = (h + sq) / a;
-    if (t <= tmin || t >= tmax) return false;
+    if (t <= tmin || (kInclusive ? t > tmax : t >= tmax)) return false;
   }
   tout = t;
   return true;
@@ -155,6 +156,7 @@ ZT_D void sphere_hit(dv3 center, double radius, uint32_t mat, dv3 o, dv3 d, doub
 }
 
 /* Moller-Trumbore, geometry.zig:83-99, with e1/e2 precomputed. */
+template <bool kInclusive = false>
 ZT_D bool triangle_t(dv3 v0, dv3 e1, dv3 e2, dv3 o, dv3 d, double tmin, double tmax, double& tout) {
   const dv3 p = vcross(d, e2);
   const double det = vdot(e1, p);
@@ -167,7 +169,7 @@ ZT_D bool triangle_t(dv3 v0, dv3 e1, dv3 e2, dv3 o, dv3 d, double tmin, double t
   const double v = vdot(d, q) * inv_det;
   if (v < 0 || u + v > 1) return false;
   const double t = vdot(e2, q) * inv_det;
-  if (t <= tmin || t >= tmax) return false;
+  if (t <= tmin || (kInclusive ? t > tmax : t >= tmax)) return false;
   tout = t;
   return true;
 }
@@ -192,14 +194,15 @@ ZT_D bool plane_t(dv3 point, dv3 normal, dv3 o, dv3 d, double tmin, double tmax,
  * faster on the 1M-triangle terrain (where shadow rays are half the frame)
  * and the same elsewhere; both give the same answer for every primitive of
  * the tree. */
+template <bool kInclusive = false>
 ZT_D bool bounded_t(const DPrim& pg, dv3 o, dv3 d, double tmin, double tmax, double& t) {
   /* five 16-byte read-only loads of the 80-byte record */
   const double2* q = reinterpret_cast<const double2*>(&pg);
   const double2 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3), q4 = __ldg(q + 4);
   const uint32_t kind = (uint32_t)((unsigned long long)__double_as_longlong(q4.y) >> 32); /* material, kind */
   if (kind == kTriangle)
-    return triangle_t(V(q0.x, q0.y, q1.x), V(q1.y, q2.x, q2.y), V(q3.x, q3.y, q4.x), o, d, tmin, tmax, t);
-  return sphere_t(V(q0.x, q0.y, q1.x), q1.y, o, d, tmin, tmax, t);
+    return triangle_t<kInclusive>(V(q0.x, q0.y, q1.x), V(q1.y, q2.x, q2.y), V(q3.x, q3.y, q4.x), o, d, tmin, tmax, t);
+  return sphere_t<kInclusive>(V(q0.x, q0.y, q1.x), q1.y, o, d, tmin, tmax, t);
 }
 /* Any primitive kind (the any-hit walks' leaf and plane loops). */
 ZT_D bool prim_t(const DPrim& pg, dv3 o, dv3 d, double tmin, double tmax, double& t) {
@@ -438,16 +441,23 @@ ZT_D bool scene_occluded(const DevScene& sc, dv3 o, dv3 d, double tmin, double t
 
 namespace zt {
 
-/* Closest or any hit with the hit record (kAnyHit: t only).  kFast walks
- * the float records (zt_fast.cuh) for closest-hit queries. */
-template <bool kAnyHit, bool kFast = false>
-ZT_D bool scene_intersect(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax, Hit& out) {
+/* How a kernel instance walks the tree.  kWalkFloatChecked is the float walk
+ * with every hit checked against what the f64 walk would find; where that
+ * cannot be shown it sets `unsure`, and the caller renders the pixel again
+ * with the f64 walk. */
+enum Walk : int { kWalkF64 = 0, kWalkFloat = 1, kWalkFloatChecked = 2 };
+
+/* Closest hit with the hit record. */
+template <int kWalk>
+ZT_D bool scene_intersect(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax, Hit& out, bool& unsure) {
   double t;
-  const int32_t k = (kFast && !kAnyHit) ? scene_query_fast(sc, o, d, tmin, tmax, t)
-                                        : scene_query<kAnyHit>(sc, o, d, tmin, tmax, t);
+  const int32_t k = kWalk != kWalkF64
+                        ? scene_query_fast<kWalk == kWalkFloatChecked>(sc, o, d, tmin, tmax, t, unsure)
+                        : scene_query<false>(sc, o, d, tmin, tmax, t);
   if (k == -1) return false;
   out.t = t;
-  if (!kAnyHit) hit_from(sc, k, o, d, t, out);
+  hit_from(sc, k, o, d, t, out);
+  if (kWalk == kWalkFloatChecked && k >= 0 && !walk_reaches(sc, sc.prims[k], o, out.point)) unsure = true;
   return true;
 }
 
@@ -660,18 +670,18 @@ ZT_D double power_weight(double a, double b) { /* render.zig:38-41 */
   return a2 / (a2 + b * b);
 }
 
-/* directLight, render.zig:46-56 (shadow ray as an any-hit query; kFast
- * walks the float records). */
-template <bool kFast = false>
-ZT_D dv3 direct_light(const DevScene& sc, dv3 albedo, const Hit& hit, Rng& rng) {
+/* directLight, render.zig:46-56 (shadow ray as an any-hit query). */
+template <int kWalk>
+ZT_D dv3 direct_light(const DevScene& sc, dv3 albedo, const Hit& hit, Rng& rng, bool& unsure) {
   dv3 ldir, lrad;
   double ldist, lpdf;
-  if (!lights_sample<kFast>(sc, hit.point, rng, ldir, ldist, lrad, lpdf)) return V(0, 0, 0);
+  if (!lights_sample<kWalk != kWalkF64>(sc, hit.point, rng, ldir, ldist, lrad, lpdf)) return V(0, 0, 0);
   const double cos_s = vdot(hit.normal, ldir);
   if (cos_s <= 0 || !(lpdf > 0)) return V(0, 0, 0);
   const double shadow_tmax = ldist * (1 - 1e-6);
-  if (kFast ? scene_occluded_fast(sc, hit.point, ldir, kRayEpsilon, shadow_tmax)
-            : scene_occluded(sc, hit.point, ldir, kRayEpsilon, shadow_tmax))
+  if (kWalk != kWalkF64
+          ? scene_occluded_fast<kWalk == kWalkFloatChecked>(sc, hit.point, ldir, kRayEpsilon, shadow_tmax, unsure)
+          : scene_occluded(sc, hit.point, ldir, kRayEpsilon, shadow_tmax))
     return V(0, 0, 0);
   const double bsdf_pdf = cos_s / kPi;
   const double scale = cos_s / (kPi * lpdf) * power_weight(lpdf, bsdf_pdf);
@@ -683,9 +693,9 @@ ZT_D dv3 direct_light(const DevScene& sc, dv3 albedo, const Hit& hit, Rng& rng) 
  * path is then the reference's use_nee = false path, draw for draw. */
 struct TraceAux { int32_t first_prim; uint32_t path_len; };
 
-template <bool kAux, bool kNee = true, bool kFast = false>
+template <bool kAux, bool kNee, int kWalk>
 ZT_D dv3 trace_with(const DevScene& sc, dv3 ro, dv3 rd, Rng& rng, uint64_t max_depth, bool use_nee_arg,
-                    TraceAux* aux) {
+                    TraceAux* aux, bool& unsure) {
   const bool use_nee = kNee && use_nee_arg;
   /* The reference's prev_origin (render.zig:66-70) is read only when
    * prev_pdf > 0, i.e. after a bounce, where it always equals the current
@@ -698,7 +708,7 @@ ZT_D dv3 trace_with(const DevScene& sc, dv3 ro, dv3 rd, Rng& rng, uint64_t max_d
   for (uint64_t depth = 0; depth < max_depth; ++depth) {
     Hit hit;
     if (kAux) n_ext++;
-    if (!scene_intersect<false, kFast>(sc, ro, rd, kRayEpsilon, INFINITY, hit)) {
+    if (!scene_intersect<kWalk>(sc, ro, rd, kRayEpsilon, INFINITY, hit, unsure)) {
       if (kAux) aux->path_len = n_ext;
       return radiance + vmul(throughput, background_radiance(sc.bg, rd));
     }
@@ -707,11 +717,11 @@ ZT_D dv3 trace_with(const DevScene& sc, dv3 ro, dv3 rd, Rng& rng, uint64_t max_d
     /* Material.emitted, material.zig:26-32 */
     const dv3 le = (mat.kind == kEmissive && hit.front_face) ? L3(mat.color) : V(0, 0, 0);
     if (vmaxc(le) > 0) {
-      const double w = prev_pdf > 0 ? power_weight(prev_pdf, lights_pdf_hit<kFast>(sc, ro, hit.point)) : 1.0;
+      const double w = prev_pdf > 0 ? power_weight(prev_pdf, lights_pdf_hit<kWalk != kWalkF64>(sc, ro, hit.point)) : 1.0;
       radiance = radiance + vscale(vmul(throughput, le), w);
     }
     if (mat.kind == kLambertian && use_nee)
-      radiance = radiance + vmul(throughput, direct_light<kFast>(sc, L3(mat.color), hit, rng));
+      radiance = radiance + vmul(throughput, direct_light<kWalk>(sc, L3(mat.color), hit, rng, unsure));
     dv3 atten, sd;
     if (!material_scatter(mat, rd, hit, rng, atten, sd)) break;
     throughput = vmul(throughput, atten);

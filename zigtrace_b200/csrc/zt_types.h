@@ -126,6 +126,8 @@ struct DevScene {
   float froot[3][2]; /* root box, [axis][lower, upper] as in FPair */
   uint32_t froot_word;
   uint32_t fast_ok;   /* 1 when the fast records exist (leaves <= 15 primitives, bounds within kFastMaxCoord) */
+  float freach;       /* largest |bound| of the root box, rounded up */
+  uint32_t verify_ok; /* 1 when the float walk's hits can be checked against the f64 walk (walk_reaches) */
 };
 
 struct RenderParams {
