@@ -77,3 +77,20 @@ def test_encode_counts_and_alignment(pixels, offset):
     want = zt.Image(pixels, 1, v.reshape(-1, 3)).to_rgb8()
     assert (got[offset[1]:offset[1] + 3 * pixels] == want).all()
     assert (got[:offset[1]] == 77).all() and (got[offset[1] + 3 * pixels:] == 77).all()
+
+
+@pytest.mark.parametrize("offset", [(0, 0), (1, 0), (2, 5), (3, 31), (0, 16)])
+@pytest.mark.parametrize("w,h", [(1, 1), (2, 3), (10, 1), (11, 2), (43, 61), (107, 25), (2720, 1), (2721, 1),
+                                 (21845, 1), (21846, 2), (300, 219)])
+def test_png_sizes_and_alignment(w, h, offset):
+    import torch
+    rng = np.random.default_rng(w + h)
+    rgb = rng.integers(0, 256, 3 * w * h).astype(np.uint8)
+    want = np.frombuffer(zt.encode_png(rgb, w, h), np.uint8)
+    d = torch.zeros(3 * w * h + 4, dtype=torch.uint8, device="cuda")
+    d[offset[0]:offset[0] + len(rgb)] = torch.from_numpy(rgb).cuda()
+    out = torch.full((len(want) + 64,), 77, dtype=torch.uint8, device="cuda")
+    zt.encode_png_device(d.data_ptr() + offset[0], w, h, out.data_ptr() + offset[1], len(want))
+    got = out.cpu().numpy()
+    assert (got[offset[1]:offset[1] + len(want)] == want).all()
+    assert (got[:offset[1]] == 77).all() and (got[offset[1] + len(want):] == 77).all()

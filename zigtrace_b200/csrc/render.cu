@@ -123,7 +123,7 @@ static zt_status device_pool(cudaMemPool_t* out) {
   return ZT_OK;
 }
 
-static zt_status pool_alloc(void** p, size_t bytes, cudaStream_t st, const char* what) {
+zt_status pool_alloc(void** p, size_t bytes, cudaStream_t st, const char* what) {
   cudaMemPool_t pool = nullptr;
   zt_status rc = device_pool(&pool);
   if (rc != ZT_OK) return rc;
