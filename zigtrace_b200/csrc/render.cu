@@ -36,7 +36,7 @@ struct zt_host_staging {
   void* pinned = nullptr;
   size_t bytes = 0;
   size_t off_prims = 0, off_ids = 0, off_pairs = 0, off_fpairs = 0, off_planes = 0, off_mats = 0, off_lights = 0,
-         off_cdf = 0;
+         off_flights = 0, off_cdf = 0;
   DevScene view;  /* counts, root, total; pointers unset */
 };
 
@@ -195,6 +195,7 @@ static zt_status make_staging(zt_scene* s) {
   stage(f.planes, cur, h->off_planes);
   stage(f.mats, cur, h->off_mats);
   stage(f.lights, cur, h->off_lights);
+  stage(f.flights, cur, h->off_flights);
   stage(f.cdf, cur, h->off_cdf);
   h->bytes = cur > 0 ? cur : 256;
   cudaError_t e = cudaMallocHost(&h->pinned, h->bytes);
@@ -210,6 +211,7 @@ static zt_status make_staging(zt_scene* s) {
   stage_copy(f.planes, h->pinned, h->off_planes);
   stage_copy(f.mats, h->pinned, h->off_mats);
   stage_copy(f.lights, h->pinned, h->off_lights);
+  stage_copy(f.flights, h->pinned, h->off_flights);
   stage_copy(f.cdf, h->pinned, h->off_cdf);
   h->view = f.view;
   s->staging = h;
@@ -256,6 +258,7 @@ static zt_status upload(zt_scene* s, bool sync = true) {
   d->view.planes = (const DPrim*)(b + h->off_planes);
   d->view.mats = (const DMat*)(b + h->off_mats);
   d->view.lights = (const DLight*)(b + h->off_lights);
+  d->view.flights = (const FLight*)(b + h->off_flights);
   d->view.cdf = (const double*)(b + h->off_cdf);
   return s->pilot_valid ? ZT_OK : pilot_paths(s);
 }

@@ -532,6 +532,37 @@ static void make_fast_records(const zt_scene* s, FlatScene* f) {
   v.verify_ok = s->boxes_nested && !nan;
 }
 
+/* The record by which Lights.pdfHit passes a triangle light over (the margins
+ * are derived at light_passed, zt_device.cuh).  Slivers and lights out of
+ * float's comfortable range keep infinite bounds. */
+static FLight pass_over_record(const DLight& L) {
+  FLight r;
+  memset(&r, 0, sizeof r);
+  for (int k = 0; k < 3; ++k) { r.lo[k] = -INFINITY; r.hi[k] = INFINITY; }
+  if (L.kind != ZT_TRIANGLE) return r;
+  double lo[3], hi[3], reach = 0, e[3] = {0, 0, 0};
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = fmin(L.v[k], fmin(L.v[3 + k], L.v[6 + k]));
+    hi[k] = fmax(L.v[k], fmax(L.v[3 + k], L.v[6 + k]));
+    reach = fmax(reach, fmax(fabs(lo[k]), fabs(hi[k])));
+    for (int j = 0; j < 3; ++j) {
+      const double d = L.v[3 * ((j + 1) % 3) + k] - L.v[3 * j + k];
+      e[j] += d * d;
+    }
+  }
+  const double emax = sqrt(fmax(e[0], fmax(e[1], e[2])));
+  if (!(reach <= kFastMaxCoord) || !(emax >= 1e-7) || !(sqrt(e[0] * e[2]) <= 1e3 * 2 * L.area)) return r;
+  const double pad = std::ldexp(reach, -21) + 2e-7 * emax;
+  for (int k = 0; k < 3; ++k) {
+    r.lo[k] = f32_down(lo[k] - pad);
+    r.hi[k] = f32_up(hi[k] + pad);
+  }
+  r.nx = (float)L.normal[0];
+  r.ny = (float)L.normal[1];
+  r.nz = (float)L.normal[2];
+  return r;
+}
+
 void flatten_scene(const zt_scene* s, FlatScene* f) {
   const size_t n = s->shapes.size();
   f->prims.resize(n);
@@ -596,6 +627,8 @@ void flatten_scene(const zt_scene* s, FlatScene* f) {
       for (int k = 0; k < 3; ++k) d.normal[k] = nrm[k];
     }
   }
+  f->flights.resize(f->lights.size());
+  for (size_t i = 0; i < f->lights.size(); ++i) f->flights[i] = pass_over_record(f->lights[i]);
   f->cdf = s->cdf;
   v.n_prims = (uint32_t)n;
   v.n_planes = (uint32_t)s->planes.size();

@@ -37,6 +37,7 @@ struct FlatScene {
   std::vector<DPrim> planes;
   std::vector<DMat> mats;
   std::vector<DLight> lights;
+  std::vector<FLight> flights;
   std::vector<double> cdf;
   DevScene view;  /* pointers unset; counts, root, total, background set */
 };

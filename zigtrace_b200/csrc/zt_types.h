@@ -94,6 +94,15 @@ struct ZT_ALIGN(16) DLight {
   uint32_t material; /* the emitter's material (differentiable form) */
 };
 
+/* What Lights.pdfHit needs to pass a light over (zt_device.cuh, light_passed):
+ * a triangle light's bounds widened by the margins derived there, and its
+ * unit normal.  Lights that are never passed over have infinite bounds. */
+struct ZT_ALIGN(16) FLight {
+  float lo[3], nx;
+  float hi[3], ny;
+  float nz, pad[3];
+};
+
 struct DCamera {
   double origin[3], upper_left[3], horizontal[3], vertical[3], u[3], v[3];
   double lens_radius;
@@ -128,6 +137,7 @@ struct DevScene {
   uint32_t fast_ok;   /* 1 when the fast records exist (leaves <= 15 primitives, bounds within kFastMaxCoord) */
   float freach;       /* largest |bound| of the root box, rounded up */
   uint32_t verify_ok; /* 1 when the float walk's hits can be checked against the f64 walk (walk_reaches) */
+  const FLight* flights; /* one per light */
 };
 
 struct RenderParams {
