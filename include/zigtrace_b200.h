@@ -174,8 +174,10 @@ zt_status zt_scene_bvh_depth(const zt_scene* scene, uint64_t* depth_out);
  * changed, destroyed, or zt_scene_release_device is called). */
 zt_status zt_scene_upload(zt_scene* scene);
 zt_status zt_scene_release_device(zt_scene* scene);
-/* Bytes one upload copies host-to-device (the flattened scene is kept in
- * pinned host memory after the first upload, so re-uploads are one copy). */
+/* Bytes of the flattened scene on the device.  The first upload of a build
+ * flattens it there (a device build's tree is used where it lies); a second
+ * one keeps a pinned host image, so that later uploads are one copy of this
+ * many bytes. */
 zt_status zt_scene_upload_bytes(zt_scene* scene, uint64_t* bytes);
 
 /* ---- Rendering (src/render.zig:152-180) -------------------------------- */

@@ -371,7 +371,8 @@ class Scene:
         N.check(N.lib().zt_scene_set_primal_cache_limit(self.handle, int(max_bytes)))
 
     def staging_bytes(self) -> int:
-        """Bytes one upload copies host-to-device (from pinned memory)."""
+        """Bytes of the flattened scene, which a repeated upload copies
+        host-to-device from pinned memory."""
         b = C.c_uint64()
         N.check(N.lib().zt_scene_upload_bytes(self.handle, C.byref(b)))
         return b.value

@@ -45,10 +45,18 @@
 #include <string.h>
 
 #include <algorithm>
+#include <new>
 #include <string>
 #include <vector>
 
+#include "output.cuh"
 #include "scene_host.h"
+
+struct zt_device_tree {
+  int device = -1;
+  void* mem = nullptr; /* from the pool */
+  zt::DeviceTree t{};
+};
 
 namespace zt {
 
@@ -768,7 +776,109 @@ __global__ void k_emit_small(const Subtree* __restrict__ subs, uint32_t n_subs, 
   }
 }
 
+/* ------------------------------------------------------------------------
+ * The device layout (zt_types.h) from shapes, permutation and nodes.
+ * ---------------------------------------------------------------------- */
+/* One thread per primitive: gathered by the permutation, edges of triangles
+ * subtracted as the host does (flatten_scene's to_prim). */
+__global__ void __launch_bounds__(256) k_flat_prims(const zt_shape* __restrict__ shapes,
+                                                    const uint32_t* __restrict__ idx, uint32_t n,
+                                                    DPrim* __restrict__ prims, int32_t* __restrict__ ids,
+                                                    uint32_t* __restrict__ flags) {
+  const uint32_t k = blockIdx.x * 256 + threadIdx.x;
+  if (k >= n) return;
+  const uint32_t i = idx[k];
+  zt_shape s;
+  const uint4* src = reinterpret_cast<const uint4*>(shapes + i);
+  uint4* tmp = reinterpret_cast<uint4*>(&s);
+#pragma unroll
+  for (int j = 0; j < 5; ++j) tmp[j] = __ldg(src + j);
+  DPrim p;
+  p.material = s.material;
+  p.kind = s.kind;
+  double sum = 0;
+#pragma unroll
+  for (int j = 0; j < 9; ++j) {
+    p.a[j] = s.kind == ZT_TRIANGLE && j >= 3 ? s.p[j] - s.p[j % 3] : s.p[j];
+    sum += p.a[j];
+  }
+  if (isnan(sum)) atomicOr(flags + 1, 1u);
+  uint4* dst = reinterpret_cast<uint4*>(prims + k);
+  const uint4* out = reinterpret_cast<const uint4*>(&p);
+#pragma unroll
+  for (int j = 0; j < 5; ++j) dst[j] = out[j];
+  ids[k] = (int32_t)i;
+}
+
+/* One thread per pair record r: reference nodes 2r+1 and 2r+2. */
+__global__ void __launch_bounds__(256) k_flat_pairs(const HostNode* __restrict__ nodes, uint32_t n_pairs, double ex,
+                                                    double ey, double ez, DPair* __restrict__ pairs,
+                                                    FPair* __restrict__ fpairs, uint32_t* __restrict__ flags) {
+  const uint32_t r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= n_pairs) return;
+  const double eps[3] = {ex, ey, ez};
+  DPair p;
+  FPair f;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const HostNode& nd = nodes[2 * (size_t)r + 1 + c];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      p.lo[c][k] = nd.bmin[k];
+      p.hi[c][k] = nd.bmax[k];
+      f.b[c][k][0] = __double2float_rd(nd.bmin[k] - eps[k]);
+      f.b[c][k][1] = __double2float_ru(nd.bmax[k] + eps[k]);
+    }
+    p.first[c] = nd.count > 0 ? nd.first : (nd.first - 1) / 2;
+    p.count[c] = nd.count;
+    f.word[c] = nd.count << kFastCountShift | p.first[c];
+    f.pad[c] = 0;
+    if (nd.count > kFastMaxLeaf) atomicMax(flags, nd.count);
+  }
+  pairs[r] = p;
+  if (fpairs) fpairs[r] = f;
+}
+
 }  // namespace
+
+void release_device_tree(zt_scene* s) {
+  zt_device_tree* d = s->device_tree;
+  if (!d) return;
+  int cur = -1;
+  cudaGetDevice(&cur);
+  if (d->device != cur) cudaSetDevice(d->device);
+  cudaFreeAsync(d->mem, 0);
+  if (d->device != cur) cudaSetDevice(cur);
+  delete d;
+  s->device_tree = nullptr;
+}
+
+bool device_tree(const zt_scene* s, DeviceTree* out) {
+  int cur = -1;
+  if (!s->device_tree || cudaGetDevice(&cur) != cudaSuccess || cur != s->device_tree->device) return false;
+  *out = s->device_tree->t;
+  return true;
+}
+
+zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_nodes, const double eps[3], DPrim* prims,
+                            int32_t* ids, DPair* pairs, FPair* fpairs, uint32_t* max_leaf, bool* nan) {
+  uint32_t* flags = nullptr;
+  zt_status rc = pool_alloc((void**)&flags, 2 * sizeof(uint32_t), 0, "flatten: flags");
+  if (rc != ZT_OK) return rc;
+  uint32_t got[2] = {0, 0};
+  cudaError_t e = cudaMemsetAsync(flags, 0, sizeof got, 0);
+  if (e == cudaSuccess && n_prims) k_flat_prims<<<(n_prims + 255) / 256, 256>>>(t.shapes, t.indices, n_prims, prims, ids, flags);
+  const uint32_t n_pairs = n_nodes / 2;
+  if (e == cudaSuccess && n_pairs)
+    k_flat_pairs<<<(n_pairs + 255) / 256, 256>>>(t.nodes, n_pairs, eps[0], eps[1], eps[2], pairs, fpairs, flags);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpy(got, flags, sizeof got, cudaMemcpyDeviceToHost);
+  cudaFreeAsync(flags, 0);
+  if (e != cudaSuccess) return fail(ZT_ERR_CUDA, std::string("flatten the scene: ") + cudaGetErrorString(e));
+  *max_leaf = got[0];
+  *nan = got[1] != 0;
+  return ZT_OK;
+}
 
 /* Host driver.  Returns ZT_OK with s->nodes / s->indices filled, or
  * ZT_DEVICE_BUILD_FALLBACK when the host builder must be used. */
@@ -784,12 +894,15 @@ zt_status device_build_bvh(zt_scene* s, double* build_ms) {
   cudaEventCreate(&ev1);
   cudaEventRecord(ev0, 0);
 
-  /* one allocation for everything */
+  /* one allocation for what the flattening reads as well (shapes,
+   * permutation, nodes; kept until the scene is uploaded), one for
+   * everything else */
   const uint32_t max_large = 2 * (N / (kSmall + 1)) + 2;
   const uint32_t max_subs = 2 * max_large + 2;
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
   size_t off = 0;
-  const size_t o_shapes = off; off += up(n * sizeof(zt_shape));
+  const size_t k_shapes = 0, k_idx = up(n * sizeof(zt_shape)), k_out = k_idx + up(n * 4);
+  const size_t k_bytes = k_out + up((2 * n - 1) * sizeof(HostNode));
   const size_t o_boxes = off; off += up(n * sizeof(DBox));
   const size_t o_cent = off; off += up(3 * n * sizeof(double));
   const size_t o_idx = off; off += up(n * 4);
@@ -806,16 +919,16 @@ zt_status device_build_bvh(zt_scene* s, double* build_ms) {
   const size_t o_ctl = off; off += up(16 * 4);
   const size_t o_acc = off; off += up((size_t)(N / (kSmall + 1) + 1) * kAcc * 8);
   const size_t o_lnodes = off; off += up(2 * n * sizeof(LNode));
-  const size_t o_out = off; off += up((2 * n - 1) * sizeof(HostNode));
-  unsigned char* mem = nullptr;
-  cudaError_t e = cudaMalloc((void**)&mem, off);
-  if (e != cudaSuccess) { /* no device, or not enough device memory: the host builds it */
+  unsigned char *mem = nullptr, *kept = nullptr;
+  if (pool_alloc((void**)&kept, k_bytes, 0, "device BVH build") != ZT_OK ||
+      pool_alloc((void**)&mem, off, 0, "device BVH build") != ZT_OK) { /* no device, or not enough device memory: the host builds it */
+    if (kept) cudaFreeAsync(kept, 0);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
     cudaGetLastError();
     return ZT_DEVICE_BUILD_FALLBACK;
   }
-  zt_shape* d_shapes = (zt_shape*)(mem + o_shapes);
+  zt_shape* d_shapes = (zt_shape*)(kept + k_shapes);
   DBox* d_boxes = (DBox*)(mem + o_boxes);
   double* d_cent = (double*)(mem + o_cent);
   uint32_t* d_idx = (uint32_t*)(mem + o_idx);
@@ -832,7 +945,7 @@ zt_status device_build_bvh(zt_scene* s, double* build_ms) {
   uint32_t* d_ctl = (uint32_t*)(mem + o_ctl); /* 0 n_large, 1 n_next, 2 n_subs, 3 bad, 4 fallback */
   u64* d_acc = (u64*)(mem + o_acc);
   LNode* d_lnodes = (LNode*)(mem + o_lnodes);
-  HostNode* d_out = (HostNode*)(mem + o_out);
+  HostNode* d_out = (HostNode*)(kept + k_out);
 
   zt_status rc = ZT_OK;
   auto ck = [&](cudaError_t err, const char* what) {
@@ -950,7 +1063,20 @@ zt_status device_build_bvh(zt_scene* s, double* build_ms) {
     cudaEventElapsedTime(&ms, ev0, ev1);
     *build_ms = ms;
   }
-  cudaFree(mem);
+  if (rc == ZT_OK) {
+    zt_device_tree* d = new (std::nothrow) zt_device_tree();
+    if (d && cudaGetDevice(&d->device) == cudaSuccess &&
+        cudaMemcpyAsync(kept + k_idx, d_idx, n * 4, cudaMemcpyDeviceToDevice, 0) == cudaSuccess) {
+      d->mem = kept;
+      d->t = DeviceTree{d_shapes, (uint32_t*)(kept + k_idx), d_out};
+      s->device_tree = d;
+      kept = nullptr;
+    } else {
+      delete d;
+    }
+  }
+  if (kept) cudaFreeAsync(kept, 0);
+  cudaFreeAsync(mem, 0);
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
   if (rc != ZT_OK) {

@@ -268,6 +268,7 @@ zt_status build_scene(zt_scene* s, bool device, bool* used_device, double* build
   for (const zt_shape& sh : s->planes)
     if (sh.material >= s->materials.size()) return fail(ZT_ERR_INVALID_ARGUMENT, "plane refers to an undefined material");
   release_staging(s);
+  release_device_tree(s);
   s->built = false;
   s->pilot_valid = false;
   zt_status rc;
@@ -371,6 +372,7 @@ zt_status import_bvh(zt_scene* s, const zt_bvh_node* nodes, size_t n_nodes, cons
   for (size_t k = 0; k < n; ++k)
     if (!covered[k]) return bad("shape position " + std::to_string(k) + " is in no leaf");
   release_staging(s);
+  release_device_tree(s);
   s->built = false;
   s->pilot_valid = false;
   try {
@@ -478,26 +480,27 @@ static float f32_up(double x) {
  * also reaches its float copy.  Left empty (fast traversal unavailable) when
  * a leaf holds more than kFastMaxLeaf primitives, the tree is too large for
  * the packed payload word, or the bounds exceed kFastMaxCoord. */
-static void make_fast_records(const zt_scene* s, FlatScene* f) {
+static void make_fast_records(const zt_scene* s, FlatScene* f, bool with_tree) {
   DevScene& v = f->view;
   v.fast_ok = 0;
   f->fpairs.clear();
   const size_t nn = s->nodes.size();
-  if (nn == 0 || s->shapes.size() > kFastFirstMask || f->pairs.size() > kFastFirstMask) return;
-  double eps[3];
+  if (nn == 0 || s->shapes.size() > kFastFirstMask || nn / 2 > kFastFirstMask) return;
+  double* eps = f->fast_eps;
   for (int k = 0; k < 3; ++k) {
     const double m = std::max(std::fabs(s->nodes[0].bmin[k]), std::fabs(s->nodes[0].bmax[k]));
     if (!(m <= kFastMaxCoord)) return; /* also rejects NaN */
     eps[k] = std::ldexp(m, -20);
   }
-  for (const HostNode& nd : s->nodes)
-    if (nd.count > kFastMaxLeaf) return;
+  if (with_tree)
+    for (const HostNode& nd : s->nodes)
+      if (nd.count > kFastMaxLeaf) return;
   auto word = [&](uint32_t c) -> uint32_t {
     const HostNode& nd = s->nodes[c];
     return nd.count > 0 ? (nd.count << kFastCountShift) | nd.first : (nd.first - 1) / 2;
   };
-  f->fpairs.assign(f->pairs.size(), FPair{});
-  for (size_t i = 0; i < nn; ++i) {
+  f->fpairs.assign(f->pairs.size(), FPair{}); /* none without the tree */
+  for (size_t i = 0; with_tree && i < nn; ++i) {
     const HostNode& nd = s->nodes[i];
     if (nd.count > 0) continue;
     FPair& pr = f->fpairs[(nd.first - 1) / 2];
@@ -563,24 +566,24 @@ static FLight pass_over_record(const DLight& L) {
   return r;
 }
 
-void flatten_scene(const zt_scene* s, FlatScene* f) {
+void flatten_scene(const zt_scene* s, FlatScene* f, bool with_tree) {
   const size_t n = s->shapes.size();
-  f->prims.resize(n);
-  f->prim_ids.resize(n);
-  for (size_t k = 0; k < n; ++k) {
+  f->prims.resize(with_tree ? n : 0);
+  f->prim_ids.resize(with_tree ? n : 0);
+  for (size_t k = 0; with_tree && k < n; ++k) {
     f->prims[k] = to_prim(s->shapes[s->indices[k]]);
     f->prim_ids[k] = (int32_t)s->indices[k];
   }
   DevScene& v = f->view;
   memset(&v, 0, sizeof v);
   const size_t nn = s->nodes.size();
-  f->pairs.assign(nn > 1 ? (nn - 1) / 2 : 0, DPair{});
+  f->pairs.assign(with_tree && nn > 1 ? (nn - 1) / 2 : 0, DPair{});
   auto payload = [&](uint32_t c, uint32_t& first, uint32_t& count) {
     const HostNode& nd = s->nodes[c];
     if (nd.count > 0) { first = nd.first; count = nd.count; }
     else { first = (nd.first - 1) / 2; count = 0; }
   };
-  for (size_t i = 0; i < nn; ++i) {
+  for (size_t i = 0; with_tree && i < nn; ++i) {
     const HostNode& nd = s->nodes[i];
     if (nd.count > 0) continue;
     DPair& pr = f->pairs[(nd.first - 1) / 2];
@@ -595,7 +598,7 @@ void flatten_scene(const zt_scene* s, FlatScene* f) {
     for (int k = 0; k < 3; ++k) { v.root_lo[k] = s->nodes[0].bmin[k]; v.root_hi[k] = s->nodes[0].bmax[k]; }
     payload(0, v.root_first, v.root_count);
   }
-  make_fast_records(s, f);
+  make_fast_records(s, f, with_tree);
   f->planes.resize(s->planes.size());
   for (size_t i = 0; i < s->planes.size(); ++i) f->planes[i] = to_prim(s->planes[i]);
   f->mats.resize(s->materials.size());
@@ -667,6 +670,7 @@ zt_status zt_scene_create(zt_scene** out) { /* Scene.init, scene.zig:53-55 */
 void zt_scene_destroy(zt_scene* s) {
   if (!s) return;
   release_staging(s);
+  release_device_tree(s);
   delete s;
 }
 
@@ -701,6 +705,7 @@ zt_status zt_scene_add_shapes(zt_scene* s, const zt_shape* shapes, size_t n) { /
   for (size_t i = 0; i < n; ++i)
     if (shapes[i].kind > ZT_PLANE) return fail(ZT_ERR_INVALID_ARGUMENT, "unknown shape kind");
   release_staging(s);
+  release_device_tree(s);
   s->built = false; /* Scene.invalidate, scene.zig:98-102 */
   try {
     for (size_t i = 0; i < n; ++i) {

@@ -12,7 +12,8 @@
 #include "../../include/zigtrace_b200.h"
 #include "zt_types.h"
 
-struct zt_device_buffers;  /* defined by the CUDA side */
+struct zt_device_buffers;
+struct zt_device_tree;  /* defined by the CUDA side */
 struct zt_host_staging;    /* pinned flattened copy, defined by the CUDA side */
 
 namespace zt {
@@ -39,6 +40,7 @@ struct FlatScene {
   std::vector<DLight> lights;
   std::vector<FLight> flights;
   std::vector<double> cdf;
+  double fast_eps[3]; /* margins of the float records */
   DevScene view;  /* pointers unset; counts, root, total, background set */
 };
 
@@ -61,6 +63,8 @@ struct zt_scene {
   bool pilot_valid = false;             /* mean_path is current for this build, camera and background */
   double mean_path = 0;                 /* mean path length of the pilot that ZT_MODE_AUTO reads */
   zt_host_staging* staging = nullptr;   /* pinned flattened copy, owned */
+  zt_device_tree* device_tree = nullptr; /* shapes and tree left on the device by a device build, owned */
+  bool uploaded = false;                /* since the last build */
   uint64_t primal_cache_limit = 1ull << 30; /* bytes zt_forward may keep for zt_backward */
 };
 
@@ -81,8 +85,26 @@ constexpr zt_status ZT_DEVICE_BUILD_FALLBACK = 1;
 zt_status device_build_bvh(zt_scene* s, double* build_ms);
 /* Camera.init (camera.zig:29-55) for the given aspect ratio. */
 DCamera camera_init(const zt_camera_config& cfg, double aspect);
-/* Flattens a built scene into the device layout. */
-void flatten_scene(const zt_scene* s, FlatScene* out);
+/* Flattens a built scene into the device layout.  with_tree = false leaves
+ * prims, prim_ids, pairs and fpairs empty for the device to fill
+ * (flatten_on_device, bvh_build.cu) and sets the view's root and the float
+ * records' root and margins (fast_eps) as far as the root box decides them. */
+void flatten_scene(const zt_scene* s, FlatScene* out, bool with_tree = true);
+/* Shapes, permutation and nodes of a scene in device memory. */
+struct DeviceTree {
+  const zt_shape* shapes;
+  const uint32_t* indices;
+  const HostNode* nodes;
+};
+/* Drops what a device build left on the device. */
+void release_device_tree(zt_scene* s);
+/* The tree a device build left on the current device, if it did. */
+bool device_tree(const zt_scene* s, DeviceTree* out);
+/* Fills the tree's part of the device layout from t on the legacy default
+ * stream: the same bytes as flatten_scene's.  fpairs may be NULL.
+ * *max_leaf: the largest leaf; *nan: a primitive holds a NaN. */
+zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_nodes, const double eps[3], DPrim* prims,
+                            int32_t* ids, DPair* pairs, FPair* fpairs, uint32_t* max_leaf, bool* nan);
 /* Drops the resident device copy (implemented with the CUDA code). */
 void release_device(zt_scene* s);
 /* Drops the device copy and the pinned staging copy (scene changed). */
