@@ -14,8 +14,10 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <new>
+#include <thread>
 
 namespace zt {
 
@@ -26,6 +28,26 @@ void set_error(const std::string& msg) { g_last_error = msg; }
 zt_status fail(zt_status code, const std::string& msg) {
   g_last_error = msg;
   return code;
+}
+
+/* Calls f(begin, end) over [0, n) split among at most eight threads, the
+ * calling one included; below `grain` elements, or where no thread can be
+ * started, the caller does the work.  f must not throw. */
+template <typename F>
+static void parallel_ranges(size_t n, size_t grain, const F& f) {
+  const size_t cores = std::max(1u, std::thread::hardware_concurrency());
+  const size_t parts = std::max<size_t>(1, std::min({n / grain, cores, (size_t)8}));
+  std::thread team[8];
+  size_t started = 0;
+  try {
+    for (; started + 1 < parts; ++started) {
+      const size_t a = n * started / parts, b = n * (started + 1) / parts;
+      team[started] = std::thread([&f, a, b] { f(a, b); });
+    }
+  } catch (...) { /* fewer threads */
+  }
+  f(n * started / parts, n);
+  for (size_t i = 0; i < started; ++i) team[i].join();
 }
 
 /* ------------------------------------------------------------ AABB ---- */
@@ -85,7 +107,7 @@ constexpr size_t kMaxDepth = 64;
 constexpr double kTraversalCost = 1.0;
 
 struct Builder {
-  std::vector<HostNode>& nodes;
+  Array<HostNode>& nodes;
   uint32_t* indices;
   const std::vector<Box>& boxes;
   const std::vector<double>& cent;  /* 3 per primitive */
@@ -232,10 +254,23 @@ static inline double tri_area(const double* p) { /* light.zig:42-44 */
 
 static const double kPi = 3.14159265358979323846;
 
+constexpr size_t kEmitBlock = 1024;
+
 static zt_status build_lights(zt_scene* s) {
   s->lights.clear();
   s->cdf.clear();
-  for (const zt_shape& sh : s->shapes) {
+  /* which shapes emit: the scan reads every shape, so it is split */
+  std::vector<uint8_t> emits((s->shapes.size() + kEmitBlock - 1) / kEmitBlock, 0);
+  parallel_ranges(emits.size(), 64, [&](size_t begin, size_t end) {
+    for (size_t i = begin * kEmitBlock; i < std::min(end * kEmitBlock, s->shapes.size()); ++i)
+      if (s->materials[s->shapes[i].material].kind == ZT_EMISSIVE) emits[i / kEmitBlock] = 1;
+  });
+  for (size_t at = 0; at < s->shapes.size(); ++at) {
+    if (!emits[at / kEmitBlock]) {
+      at += kEmitBlock - 1 - at % kEmitBlock; /* the next block */
+      continue;
+    }
+    const zt_shape& sh = s->shapes[at];
     double area;
     if (sh.kind == ZT_TRIANGLE) area = tri_area(sh.p);
     else if (sh.kind == ZT_SPHERE) area = sh.p[3] > 0 ? 4 * kPi * sh.p[3] * sh.p[3] : 0;
@@ -262,11 +297,22 @@ static zt_status build_lights(zt_scene* s) {
   return ZT_OK;
 }
 
-zt_status build_scene(zt_scene* s, bool device, bool* used_device, double* build_ms) { /* Scene.build, scene.zig:92-96 */
-  for (const zt_shape& sh : s->shapes)
-    if (sh.material >= s->materials.size()) return fail(ZT_ERR_INVALID_ARGUMENT, "shape refers to an undefined material");
+static zt_status check_materials(const zt_scene* s) {
+  std::atomic<bool> bad{false};
+  parallel_ranges(s->shapes.size(), 1 << 16, [&](size_t begin, size_t end) {
+    uint32_t most = 0;
+    for (size_t i = begin; i < end; ++i) most = std::max(most, s->shapes[i].material);
+    if (end > begin && most >= s->materials.size()) bad = true;
+  });
+  if (bad) return fail(ZT_ERR_INVALID_ARGUMENT, "shape refers to an undefined material");
   for (const zt_shape& sh : s->planes)
     if (sh.material >= s->materials.size()) return fail(ZT_ERR_INVALID_ARGUMENT, "plane refers to an undefined material");
+  return ZT_OK;
+}
+
+zt_status build_scene(zt_scene* s, bool device, bool* used_device, double* build_ms) { /* Scene.build, scene.zig:92-96 */
+  const zt_status materials = check_materials(s);
+  if (materials != ZT_OK) return materials;
   release_staging(s);
   release_device_tree(s);
   s->built = false;
@@ -323,10 +369,8 @@ static bool boxes_nested(const zt_scene* s) {
  * the reference's max_depth (64), so the traversal stack of max_depth + 2
  * entries (bvh.zig:87) cannot overflow; leaves cover [0, n) exactly once. */
 zt_status import_bvh(zt_scene* s, const zt_bvh_node* nodes, size_t n_nodes, const uint32_t* indices, size_t n_idx) {
-  for (const zt_shape& sh : s->shapes)
-    if (sh.material >= s->materials.size()) return fail(ZT_ERR_INVALID_ARGUMENT, "shape refers to an undefined material");
-  for (const zt_shape& sh : s->planes)
-    if (sh.material >= s->materials.size()) return fail(ZT_ERR_INVALID_ARGUMENT, "plane refers to an undefined material");
+  const zt_status materials = check_materials(s);
+  if (materials != ZT_OK) return materials;
   const size_t n = s->shapes.size();
   auto bad = [](const std::string& why) { return fail(ZT_ERR_INVALID_ARGUMENT, "zt_scene_set_bvh: " + why); };
   if (n > 0xFFFFFFFFull / 2) return fail(ZT_ERR_TOO_MANY_PRIMITIVES, "TooManyPrimitives"); /* bvh.zig:44 */
@@ -702,12 +746,25 @@ zt_status zt_scene_add_materials(zt_scene* s, const zt_material* m, size_t n, ui
 
 zt_status zt_scene_add_shapes(zt_scene* s, const zt_shape* shapes, size_t n) { /* Scene.add */
   if (!s || (!shapes && n)) return fail(ZT_ERR_INVALID_ARGUMENT, "zt_scene_add_shapes: NULL argument");
-  for (size_t i = 0; i < n; ++i)
-    if (shapes[i].kind > ZT_PLANE) return fail(ZT_ERR_INVALID_ARGUMENT, "unknown shape kind");
+  std::atomic<uint32_t> seen{0}; /* bit k: some shape has kind k (3: an unknown one) */
+  parallel_ranges(n, 1 << 16, [&](size_t begin, size_t end) {
+    uint32_t bits = 0;
+    for (size_t i = begin; i < end; ++i) bits |= 1u << std::min<uint32_t>(shapes[i].kind, 3u);
+    seen |= bits;
+  });
+  if (seen & 8u) return fail(ZT_ERR_INVALID_ARGUMENT, "unknown shape kind");
   release_staging(s);
   release_device_tree(s);
   s->built = false; /* Scene.invalidate, scene.zig:98-102 */
   try {
+    if (!(seen & (1u << ZT_PLANE))) {
+      const size_t at = s->shapes.size();
+      s->shapes.resize(at + n); /* filled below */
+      parallel_ranges(n, 1 << 16, [&](size_t begin, size_t end) {
+        memcpy(s->shapes.data() + at + begin, shapes + begin, (end - begin) * sizeof(zt_shape));
+      });
+      return ZT_OK;
+    }
     for (size_t i = 0; i < n; ++i) {
       if (shapes[i].kind == ZT_PLANE) s->planes.push_back(shapes[i]);
       else s->shapes.push_back(shapes[i]);
