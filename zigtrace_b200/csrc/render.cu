@@ -1575,14 +1575,16 @@ zt_status zt_rng_streams(uint64_t seed, uint64_t stream0, uint64_t n_streams, ui
 /* --------------------------------------------------- Differentiable form ---- */
 namespace zt {
 
-/* Forward of the detached estimator (zt_diff.cuh): the megakernel's tile
- * loop with trace_diff; theta == the scene's colours gives zt_render's image.
- * The differentiable kernels are built for four blocks of 128 per SM (128
- * registers): their longer code spills heavily at 72 registers, and at
- * 512x512 the fewer resident warps measured faster (forward 28 vs 31 ms,
- * backward 52 vs 57-62 ms). */
+/* Forward of the detached estimator (zt_diff.cuh): the megakernel's tile loop
+ * with per-lane path regeneration (render_pixel_regen: a lane whose path ends
+ * starts its pixel's next sample at once); theta == the scene's colours gives
+ * zt_render's image.  sample_L (may be NULL) keeps every sample's radiance
+ * for zt_backward.  Built for four blocks of 128 per SM (128 registers):
+ * 512x512x64 of the Cornell-style box 25.3 ms, at five blocks 26.1, nested
+ * (every lane waiting for the warp's longest path) 28.4. */
 template <int BS>
-__global__ void __launch_bounds__(BS, 512 / BS) k_forward_diff(DevScene sc, RenderParams p,
+__global__ void __launch_bounds__(BS, 512 / BS) k_forward_diff(const __grid_constant__ DevScene sc,
+                                                             const __grid_constant__ RenderParams p,
                                                              const double* __restrict__ theta,
                                                              double* __restrict__ out, double* __restrict__ sample_L,
                                                              unsigned int* __restrict__ counter) {
@@ -1595,53 +1597,69 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_forward_diff(DevScene sc, Rend
     tile = __shfl_sync(0xffffffffu, tile, 0);
     if ((uint64_t)tile >= tiles) return;
     const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    if (x >= p.width || y >= row_end) continue;
+    const bool valid = x < p.width && y < row_end;
     const uint64_t pix = y * p.width + x;
-    Rng rng = rng_for_stream(p.seed, pix);
+    Rng rng = rng_for_stream(p.seed, valid ? pix : 0);
     dv3 sum = V(0, 0, 0);
-    for (uint64_t i = 0; i < p.spp; ++i) {
-      const double s = ((double)x + rng_float(rng)) / (double)p.width;
-      const double t = ((double)y + rng_float(rng)) / (double)p.height;
-      dv3 ro, rd;
-      camera_ray(p.cam, s, t, rng, ro, rd);
-      const dv3 c = trace_diff(sc, theta, ro, rd, rng, p.max_depth, p.use_nee != 0, false, V(0, 0, 0), V(0, 0, 0),
-                               nullptr, false);
-      if (sample_L) { /* the primal radiance of every sample, kept for zt_backward */
-        double* q = sample_L + 3 * (i * p.width * p.height + pix);
-        q[0] = c.x;
-        q[1] = c.y;
-        q[2] = c.z;
+    DiffPath s;
+    s.ro = s.rd = V(0, 0, 0);
+    diff_start(s);
+    uint64_t sample = 0, depth = 0;
+    bool done = !valid, fresh = valid;
+    for (;;) {
+      if (fresh) {
+        fresh = false;
+        const double u = ((double)x + rng_float(rng)) / (double)p.width;
+        const double v = ((double)y + rng_float(rng)) / (double)p.height;
+        camera_ray(p.cam, u, v, rng, s.ro, s.rd);
+        diff_start(s);
+        depth = 0;
       }
-      if (visfinite(c)) sum = sum + c;
+      if (__all_sync(0xffffffffu, done)) break;
+      if (done) continue;
+      const bool end = diff_bounce(sc, theta, s, depth, rng, p.use_nee != 0, false, V(0, 0, 0), V(0, 0, 0), nullptr);
+      depth += 1;
+      if (end || depth >= p.max_depth) {
+        if (sample_L) {
+          double* q = sample_L + 3 * (sample * p.width * p.height + pix);
+          q[0] = s.radiance.x;
+          q[1] = s.radiance.y;
+          q[2] = s.radiance.z;
+        }
+        if (visfinite(s.radiance)) sum = sum + s.radiance;
+        ++sample;
+        done = sample == p.spp;
+        fresh = !done;
+      }
     }
-    const dv3 px = vscale(sum, 1.0 / (double)p.spp);
-    const uint64_t o = pix - p.row0 * p.width; /* output starts at the band's first row */
-    out[3 * o + 0] = px.x;
-    out[3 * o + 1] = px.y;
-    out[3 * o + 2] = px.z;
+    if (valid) {
+      const dv3 px = vscale(sum, 1.0 / (double)p.spp);
+      const uint64_t o = pix - p.row0 * p.width; /* output starts at the band's first row */
+      out[3 * o + 0] = px.x;
+      out[3 * o + 1] = px.y;
+      out[3 * o + 2] = px.z;
+    }
   }
 }
 
-/* Path-replay adjoint: for every sample, the primal pass gives its radiance
- * L, then the same path is replayed from the saved RNG state accumulating
- * dL/dtheta into per-block shared memory (flushed once per block), or
- * straight into global memory when the parameter table is large.  Built for
- * five blocks of 128 per SM (up to 102 registers): 50.0 against 50.8 ms at
- * four blocks (128 registers) on the 512x512x64 Cornell-style workload; the
- * forward kernel stays at four (27.5 against 28.1 ms). */
-template <int BS>
-__global__ void __launch_bounds__(BS, 640 / BS) k_backward_diff(DevScene sc, RenderParams p,
+/* Path-replay adjoint: for every sample the path is replayed from the RNG
+ * stream accumulating dL/dtheta, with L the sample's radiance.  sample_L
+ * holds it from the forward; where it is NULL every sample is traced twice,
+ * the primal first, from the same stream state.  The lanes regenerate as in
+ * k_forward_diff (a primal pass starts its replay the same way).
+ * Gradients go to the warp's slice of `grad` (n_slices of n_params), which
+ * also keeps each sum short.  512x512x64 of the Cornell-style box, 108
+ * parameters: 28.8 ms at four blocks of 128 per SM, 30.5 at five, nested
+ * 39.6; without the cached radiance 60.1 ms at five blocks, 75.3 at four. */
+template <int BS, bool kCached>
+__global__ void __launch_bounds__(BS, (kCached ? 512 : 640) / BS) k_backward_diff(const __grid_constant__ DevScene sc,
+                                                              const __grid_constant__ RenderParams p,
                                                               const double* __restrict__ theta,
                                                               const double* __restrict__ dimg, double* grad,
-                                                              uint32_t n_params, int use_smem,
+                                                              uint32_t n_params, uint32_t n_slices,
                                                               const double* __restrict__ sample_L,
                                                               unsigned int* __restrict__ counter) {
-  extern __shared__ double sgrad[];
-  double* g = use_smem ? sgrad + (threadIdx.x >> 5) * n_params : grad; /* a slice per warp */
-  if (use_smem) {
-    for (uint32_t i = threadIdx.x; i < n_params * (BS / 32); i += BS) sgrad[i] = 0.0;
-    __syncthreads();
-  }
+  double* g = grad + (size_t)((blockIdx.x * (BS / 32) + threadIdx.x / 32) % n_slices) * n_params;
   const uint64_t tiles_x = (p.width + 7) / 8, tiles = tiles_x * ((p.rows + 3) / 4);
   const uint64_t row_end = p.row0 + p.rows;
   const unsigned lane = threadIdx.x & 31;
@@ -1650,56 +1668,61 @@ __global__ void __launch_bounds__(BS, 640 / BS) k_backward_diff(DevScene sc, Ren
     unsigned tile = 0;
     if (lane == 0) tile = atomicAdd(counter, 1u);
     tile = __shfl_sync(0xffffffffu, tile, 0);
-    if ((uint64_t)tile >= tiles) break;
+    if ((uint64_t)tile >= tiles) return;
     const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    if (x >= p.width || y >= row_end) continue;
+    const bool valid = x < p.width && y < row_end;
     const uint64_t pix = y * p.width + x;
     /* dL/dpixel of the band (rows row0 ..), pixel = sum * (1/spp), render.zig:144 */
-    const dv3 adj = vscale(L3(dimg + 3 * (pix - p.row0 * p.width)), inv_spp);
-    if (adj.x == 0 && adj.y == 0 && adj.z == 0) continue;
-    Rng rng = rng_for_stream(p.seed, pix);
-    for (uint64_t i = 0; i < p.spp; ++i) {
-      const double s = ((double)x + rng_float(rng)) / (double)p.width;
-      const double t = ((double)y + rng_float(rng)) / (double)p.height;
-      dv3 ro, rd;
-      camera_ray(p.cam, s, t, rng, ro, rd);
-      const Rng start = rng;
-      dv3 L = V(0, 0, 0);
-      int first_pass = 0;
-      if (sample_L) { /* the forward kept the primal radiance: replay only */
-        L = L3(sample_L + 3 * (i * p.width * p.height + pix));
-        first_pass = 1;
-        if (!visfinite(L)) { /* dropped by the forward (render.zig:142): advance the stream only */
-          Rng r = start;
-          trace_diff(sc, theta, ro, rd, r, p.max_depth, p.use_nee != 0, false, L, adj, g, use_smem);
-          rng = r;
-          continue;
+    const dv3 adj = valid ? vscale(L3(dimg + 3 * (pix - p.row0 * p.width)), inv_spp) : V(0, 0, 0);
+    bool done = adj.x == 0 && adj.y == 0 && adj.z == 0, fresh = !done, replay = kCached;
+    Rng rng = rng_for_stream(p.seed, valid ? pix : 0);
+    Rng start = rng; /* of the sample; the replay draws exactly what the primal drew */
+    dv3 L = V(0, 0, 0);
+    DiffPath s;
+    s.ro = s.rd = V(0, 0, 0);
+    diff_start(s);
+    uint64_t sample = 0, depth = 0;
+    bool live = false; /* the replay adds gradients: a sample that is not finite is dropped (render.zig:142) */
+    for (;;) {
+      if (fresh) {
+        fresh = false;
+        if (!kCached) {
+          if (replay) rng = start;
+          else start = rng;
         }
+        const double u = ((double)x + rng_float(rng)) / (double)p.width;
+        const double v = ((double)y + rng_float(rng)) / (double)p.height;
+        camera_ray(p.cam, u, v, rng, s.ro, s.rd);
+        if (kCached) L = L3(sample_L + 3 * (sample * p.width * p.height + pix));
+        live = replay && visfinite(L);
+        diff_start(s);
+        depth = 0;
       }
-#pragma unroll 1
-      for (int pass = first_pass; pass < 2; ++pass) { /* primal, then replay from the same stream state */
-        Rng r = start;
-        const dv3 v = trace_diff(sc, theta, ro, rd, r, p.max_depth, p.use_nee != 0, pass == 1, L, adj, g, use_smem);
-        if (pass == 0) {
-          L = v;
-          if (!visfinite(L)) { /* dropped by the forward (render.zig:142): no gradient */
-            rng = r;
-            break;
-          }
-        } else {
-          rng = r; /* the replay draws exactly what the primal drew */
+      if (__all_sync(0xffffffffu, done)) break;
+      if (done) continue;
+      const bool end = diff_bounce(sc, theta, s, depth, rng, p.use_nee != 0, live, L, adj, g);
+      depth += 1;
+      if (end || depth >= p.max_depth) {
+        if (!kCached) {
+          if (!replay) L = s.radiance;
+          replay = !replay;
         }
+        if (kCached || !replay) ++sample;
+        done = sample == p.spp;
+        fresh = !done;
       }
     }
   }
-  if (use_smem) { /* sum the warps' slices, then one global add per parameter and block */
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n_params; i += BS) {
-      double acc = 0.0;
-      for (int wi = 0; wi < BS / 32; ++wi) acc += sgrad[wi * n_params + i];
-      if (acc != 0.0) atomicAdd(grad + i, acc);
-    }
-  }
+}
+
+/* Sums the slices: one thread per parameter, coalesced across them. */
+__global__ void k_sum_slices(const double* __restrict__ grad, uint32_t n_params, uint32_t n_slices,
+                             double* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_params) return;
+  double acc = 0.0;
+  for (uint32_t k = 0; k < n_slices; ++k) acc += grad[(size_t)k * n_params + i];
+  out[i] = acc;
 }
 
 /* theta on the host: the caller's colours, or the scene's own. */
@@ -1852,28 +1875,30 @@ zt_status zt_backward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin,
   double *d_theta = nullptr, *d_img = nullptr, *d_grad = nullptr;
   if ((rc = upload_theta(th, &d_theta)) != ZT_OK) return rc;
   rc = pool_alloc((void**)&d_img, img_bytes, 0, "allocate image adjoint");
-  if (rc == ZT_OK) rc = pool_alloc((void**)&d_grad, n_params * sizeof(double), 0, "allocate gradients");
+  /* a slice per resident warp (at most five blocks of four warps per SM), within 64 MiB */
+  const uint32_t n_slices = (uint32_t)std::max<uint64_t>(
+      1, std::min<uint64_t>((uint64_t)sm_count() * 20, (64ull << 20) / (n_params * sizeof(double))));
+  const size_t grad_bytes = (size_t)n_slices * n_params * sizeof(double);
+  if (rc == ZT_OK) rc = pool_alloc((void**)&d_grad, grad_bytes + n_params * sizeof(double), 0, "allocate gradients");
   if (rc != ZT_OK) {
     pool_free(d_theta, 0);
     pool_free(d_img, 0);
     return rc;
   }
   cudaError_t e = cudaMemcpy(d_img, d_image, img_bytes, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemset(d_grad, 0, n_params * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_grad, 0, grad_bytes, 0);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->device->counter, 0, sizeof(unsigned int), 0);
   if (e == cudaSuccess) {
-    const size_t smem = (size_t)n_params * sizeof(double) * (128 / 32); /* one slice per warp */
-    const int use_smem = smem <= 48 * 1024 ? 1 : 0;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_backward_diff<128>, 128, use_smem ? smem : 0);
-    uint64_t blocks = (uint64_t)sm_count() * (per_sm > 0 ? per_sm : 1);
-    const uint64_t need = (p.width * p.rows + 127) / 128;
-    if (blocks > need) blocks = need;
-    k_backward_diff<128><<<(unsigned)blocks, 128, use_smem ? smem : 0>>>(
-        launch_view(s), p, d_theta, d_img, d_grad, n_params, use_smem, sample_L, s->device->counter);
+    if (sample_L)
+      k_backward_diff<128, true><<<persistent_grid(k_backward_diff<128, true>, 128, p.width * p.rows), 128>>>(
+          launch_view(s), p, d_theta, d_img, d_grad, n_params, n_slices, sample_L, s->device->counter);
+    else
+      k_backward_diff<128, false><<<persistent_grid(k_backward_diff<128, false>, 128, p.width * p.rows), 128>>>(
+          launch_view(s), p, d_theta, d_img, d_grad, n_params, n_slices, nullptr, s->device->counter);
+    k_sum_slices<<<(n_params + 127) / 128, 128>>>(d_grad, n_params, n_slices, d_grad + (size_t)n_slices * n_params);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(d_colors, d_grad, n_params * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(d_colors, d_grad + (size_t)n_slices * n_params, n_params * sizeof(double), cudaMemcpyDeviceToHost);
   pool_free(d_theta, 0);
   pool_free(d_img, 0);
   pool_free(d_grad, 0);

@@ -29,109 +29,114 @@
 
 namespace zt {
 
-/* Adds v to grad[3m..3m+2].  warp_private: grad is this warp's own slice of
- * shared memory, so the active lanes add in turn with plain loads and
- * stores (no atomics, no contention with other warps); otherwise global
- * atomics. */
-ZT_D void grad_add(double* grad, bool warp_private, uint32_t m, dv3 v) {
+/* Adds v to grad[3m..3m+2], in global memory without a returned value: the
+ * warp issues three instructions and goes on, and the L2 does the additions.
+ * (Lanes adding in turn to the warp's slice in shared memory kept the warp
+ * for a load, an add and a store per active lane: the backward took 50.0 ms
+ * that way and 39.6 with this, both without regeneration.) */
+ZT_D void grad_add(double* grad, uint32_t m, dv3 v) {
   double* q = grad + 3 * (size_t)m;
-  if (!warp_private) {
-    atomicAdd(q + 0, v.x);
-    atomicAdd(q + 1, v.y);
-    atomicAdd(q + 2, v.z);
-    return;
-  }
-  const unsigned mask = __activemask();
-  const int lane = (int)(threadIdx.x & 31);
-  for (unsigned mk = mask; mk; mk &= mk - 1) {
-    if (lane == __ffs(mk) - 1) {
-      q[0] += v.x;
-      q[1] += v.y;
-      q[2] += v.z;
-    }
-    __syncwarp(mask);
-  }
+  atomicAdd(q + 0, v.x);
+  atomicAdd(q + 1, v.y);
+  atomicAdd(q + 2, v.z);
 }
 
 /* The BVH query as a real call: the differentiable kernels are instruction-
  * cache bound when each of their queries inlines its own copy of the
- * traversal (measured: forward and backward ~22% faster outlined). */
+ * traversal (measured: forward and backward ~22% faster outlined).  One
+ * function for closest hits and shadow rays, told apart at run time, for the
+ * same reason: with a second one for shadow rays the forward took 31.2 ms
+ * against 25.3 (512x512x64), the backward 35.4 against 28.8. */
 __device__ __noinline__ int32_t scene_query_outlined(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax,
                                                      bool any_hit, double& t_out) {
   return scene_query_rt(sc, o, d, tmin, tmax, any_hit, t_out);
 }
 
-/* kAdj is a run-time flag so that the primal and the replay pass of the
+/* A path between two bounces. */
+struct DiffPath {
+  dv3 ro, rd, radiance, tp, tp0; /* tp with theta, tp0 with theta0 (the roulette's) */
+  double prev_pdf;
+};
+ZT_D void diff_start(DiffPath& s) {
+  s.radiance = V(0, 0, 0);
+  s.tp = s.tp0 = V(1, 1, 1);
+  s.prev_pdf = 0;
+}
+
+/* One iteration of traceWith's bounce loop; true when the path has ended.
+ * kAdj is a run-time flag so that the primal and the replay pass of the
  * backward kernel share one copy of this code (the kernel is instruction-
- * cache bound with two copies). */
-ZT_D dv3 trace_diff(const DevScene& sc, const double* __restrict__ theta, dv3 ro, dv3 rd, Rng& rng,
-                    uint64_t max_depth, bool use_nee, bool kAdj, dv3 L_total, dv3 adj, double* grad,
-                    bool warp_private) {
-  dv3 radiance = V(0, 0, 0), tp = V(1, 1, 1), tp0 = V(1, 1, 1);
-  /* prev_origin (render.zig:66-70) is read only after a bounce, where it
-   * equals ro: ro stands in for it, as in trace_with */
-  double prev_pdf = 0;
-  for (uint64_t depth = 0; depth < max_depth; ++depth) {
-    Hit hit;
-    double th_t;
-    const int32_t hk = scene_query_outlined(sc, ro, rd, kRayEpsilon, INFINITY, false, th_t);
-    if (hk == -1) return radiance + vmul(tp, background_radiance(sc.bg, rd));
-    hit_from(sc, hk, ro, rd, th_t, hit);
-    const uint32_t m = hit.material;
-    const DMat& mat = sc.mats[m];
-    const dv3 th = L3(theta + 3 * (size_t)m);
-    const bool emits = mat.kind == kEmissive && hit.front_face;
-    const dv3 le0 = emits ? L3(mat.color) : V(0, 0, 0);
-    if (vmaxc(le0) > 0) { /* emission with its MIS weight, render.zig:77-81 */
-      const double w = prev_pdf > 0 ? power_weight(prev_pdf, lights_pdf_hit(sc, ro, hit.point)) : 1.0;
-      if (kAdj) grad_add(grad, warp_private, m, vmul(adj, vscale(tp, w)));
-      radiance = radiance + vscale(vmul(tp, th), w);
-    }
-    if (mat.kind == kLambertian && use_nee) { /* directLight, render.zig:46-56 */
-      dv3 ldir, lrad0, direct = V(0, 0, 0);
-      double ldist, lpdf;
-      uint32_t li = 0;
-      if (lights_sample(sc, hit.point, rng, ldir, ldist, lrad0, lpdf, &li)) {
-        const double cos_s = vdot(hit.normal, ldir);
-        if (!(cos_s <= 0 || !(lpdf > 0))) {
-          double st;
-          if (scene_query_outlined(sc, hit.point, ldir, kRayEpsilon, ldist * (1 - 1e-6), true, st) == -1) {
-            const double bsdf_pdf = cos_s / kPi;
-            const double scale = cos_s / (kPi * lpdf) * power_weight(lpdf, bsdf_pdf);
-            const uint32_t lm = sc.lights[li].material;
-            const dv3 lrad = L3(theta + 3 * (size_t)lm);
-            direct = vscale(vmul(th, lrad), scale);
-            if (kAdj) {
-              grad_add(grad, warp_private, m, vmul(adj, vscale(vmul(tp, lrad), scale)));
-              grad_add(grad, warp_private, lm, vmul(adj, vscale(vmul(tp, th), scale)));
-            }
+ * cache bound with two copies).  prev_origin (render.zig:66-70) is read only
+ * after a bounce, where it equals ro: ro stands in for it, as in trace_with.
+ * Both derivatives with respect to the hit's own colour, the light sample's
+ * and that of every later term, are added at once. */
+ZT_D bool diff_bounce(const DevScene& sc, const double* __restrict__ theta, DiffPath& s, uint64_t depth, Rng& rng,
+                      bool use_nee, bool kAdj, dv3 L_total, dv3 adj, double* grad) {
+  Hit hit;
+  double th_t;
+  const int32_t hk = scene_query_outlined(sc, s.ro, s.rd, kRayEpsilon, INFINITY, false, th_t);
+  if (hk == -1) {
+    s.radiance = s.radiance + vmul(s.tp, background_radiance(sc.bg, s.rd));
+    return true;
+  }
+  hit_from(sc, hk, s.ro, s.rd, th_t, hit);
+  const uint32_t m = hit.material;
+  const DMat& mat = sc.mats[m];
+  const dv3 th = L3(theta + 3 * (size_t)m);
+  const bool emits = mat.kind == kEmissive && hit.front_face;
+  const dv3 le0 = emits ? L3(mat.color) : V(0, 0, 0);
+  if (vmaxc(le0) > 0) { /* emission with its MIS weight, render.zig:77-81 */
+    const double w = s.prev_pdf > 0 ? power_weight(s.prev_pdf, lights_pdf_hit(sc, s.ro, hit.point)) : 1.0;
+    if (kAdj) grad_add(grad, m, vmul(adj, vscale(s.tp, w)));
+    s.radiance = s.radiance + vscale(vmul(s.tp, th), w);
+  }
+  dv3 own = V(0, 0, 0); /* d/d theta[m] of the light sample and of what follows, without adj */
+  if (mat.kind == kLambertian && use_nee) { /* directLight, render.zig:46-56 */
+    dv3 ldir, lrad0, direct = V(0, 0, 0);
+    double ldist, lpdf;
+    uint32_t li = 0;
+    if (lights_sample(sc, hit.point, rng, ldir, ldist, lrad0, lpdf, &li)) {
+      const double cos_s = vdot(hit.normal, ldir);
+      if (!(cos_s <= 0 || !(lpdf > 0))) {
+        double st;
+        if (scene_query_outlined(sc, hit.point, ldir, kRayEpsilon, ldist * (1 - 1e-6), true, st) == -1) {
+          const double bsdf_pdf = cos_s / kPi;
+          const double scale = cos_s / (kPi * lpdf) * power_weight(lpdf, bsdf_pdf);
+          const uint32_t lm = sc.lights[li].material;
+          const dv3 lrad = L3(theta + 3 * (size_t)lm);
+          direct = vscale(vmul(th, lrad), scale);
+          if (kAdj) {
+            own = vscale(vmul(s.tp, lrad), scale);
+            grad_add(grad, lm, vmul(adj, vscale(vmul(s.tp, th), scale)));
           }
         }
       }
-      radiance = radiance + vmul(tp, direct);
     }
-    dv3 atten0, sd;
-    if (!material_scatter(mat, rd, hit, rng, atten0, sd)) break;
-    const bool param = mat.kind == kLambertian || mat.kind == kMetal;
-    const dv3 atten = param ? th : atten0;
-    if (kAdj && param) { /* every later term carries atten: their sum is L_total - radiance */
-      const dv3 rest = L_total - radiance;
-      grad_add(grad, warp_private, m, V(atten.x != 0 ? adj.x * rest.x / atten.x : 0.0, atten.y != 0 ? adj.y * rest.y / atten.y : 0.0,
-                          atten.z != 0 ? adj.z * rest.z / atten.z : 0.0));
-    }
-    tp = vmul(tp, atten);
-    tp0 = vmul(tp0, atten0);
-    prev_pdf = (use_nee && mat.kind == kLambertian) ? fmax(vdot(sd, hit.normal), 0.0) / kPi : 0;
-    ro = hit.point;
-    rd = sd;
-    if (depth + 1 >= kRouletteDepth) { /* roulette on the theta0 throughput */
-      const double p = fmin(vmaxc(tp0), 0.95);
-      if (p <= 0 || rng_float(rng) >= p) break;
-      tp = vdiv(tp, p);
-      tp0 = vdiv(tp0, p);
-    }
+    s.radiance = s.radiance + vmul(s.tp, direct);
   }
-  return radiance;
+  dv3 atten0, sd;
+  const bool scattered = material_scatter(mat, s.rd, hit, rng, atten0, sd);
+  const bool param = mat.kind == kLambertian || mat.kind == kMetal;
+  if (kAdj && param) { /* every later term carries theta[m]: their sum is L_total - radiance */
+    if (scattered) {
+      const dv3 rest = L_total - s.radiance;
+      own = own + V(th.x != 0 ? rest.x / th.x : 0.0, th.y != 0 ? rest.y / th.y : 0.0, th.z != 0 ? rest.z / th.z : 0.0);
+    }
+    grad_add(grad, m, vmul(adj, own));
+  }
+  if (!scattered) return true;
+  s.tp = vmul(s.tp, param ? th : atten0);
+  s.tp0 = vmul(s.tp0, atten0);
+  s.prev_pdf = (use_nee && mat.kind == kLambertian) ? fmax(vdot(sd, hit.normal), 0.0) / kPi : 0;
+  s.ro = hit.point;
+  s.rd = sd;
+  if (depth + 1 >= kRouletteDepth) { /* roulette on the theta0 throughput */
+    const double p = fmin(vmaxc(s.tp0), 0.95);
+    if (p <= 0 || rng_float(rng) >= p) return true;
+    s.tp = vdiv(s.tp, p);
+    s.tp0 = vdiv(s.tp0, p);
+  }
+  return false;
 }
 
 }  // namespace zt
