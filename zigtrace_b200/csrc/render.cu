@@ -401,7 +401,7 @@ static RenderParams make_params(const zt_scene* s, const zt_options* o) {
   p.use_nee = (o->light_sampling && !s->lights.empty()) ? 1u : 0u; /* render.zig:62 */
   p.row0 = 0;
   p.rows = o->height;
-  p.pad = 0;
+  p.split = 0;
   return p;
 }
 
@@ -445,6 +445,22 @@ __device__ __noinline__ void render_pixel_f64(const DevScene& sc, const RenderPa
   render_pixel<false, true, kWalkF64>(sc, p, pix, out, nullptr);
 }
 
+/* The pixel of this lane in work unit `unit`: every 8x4 tile is 2^p.split
+ * units, each a rectangle of the tile for the first lanes of the warp (8x4,
+ * 4x4, 4x2, 2x2, 2x1 or one pixel).  False: no pixel for this lane. */
+__device__ __forceinline__ bool unit_pixel(const RenderParams& p, uint64_t tiles_x, unsigned unit, uint64_t& x,
+                                           uint64_t& y) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned tile = unit >> p.split, part = unit & ((1u << p.split) - 1);
+  const unsigned sw = (p.split + 1) / 2, w = 3 - sw, h = 2 - (p.split - sw); /* parts per row; a part is 2^w x 2^h */
+  x = (uint64_t)(tile % tiles_x) * 8 + ((part & ((1u << sw) - 1)) << w) + (lane & ((1u << w) - 1));
+  y = p.row0 + (uint64_t)(tile / tiles_x) * 4 + ((part >> sw) << h) + (lane >> w);
+  return lane >> (w + h) == 0 && x < p.width && y < p.row0 + p.rows;
+}
+__host__ __device__ __forceinline__ uint64_t work_units(const RenderParams& p) {
+  return (((p.width + 7) / 8) * ((p.rows + 3) / 4)) << p.split;
+}
+
 /* Persistent megakernel: each warp takes an 8x4 pixel tile from the device
  * work counter until the image is exhausted (the device form of
  * Context.work's atomic tile counter, render.zig:113-119), so its camera rays
@@ -477,16 +493,16 @@ __host__ __device__ constexpr int mega_threads_per_sm(bool nee, int walk) {
 template <int BS, bool kNee, int kWalk>
 __global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kWalk) / BS)
     k_render_mega(const __grid_constant__ DevScene sc, const __grid_constant__ RenderParams p, double* __restrict__ out, unsigned int* __restrict__ counter) {
-  const uint64_t tiles_x = (p.width + 7) / 8, tiles = tiles_x * ((p.rows + 3) / 4);
-  const uint64_t row_end = p.row0 + p.rows;
+  const uint64_t tiles_x = (p.width + 7) / 8, units = work_units(p);
   const unsigned lane = threadIdx.x & 31;
   for (;;) {
-    unsigned tile = 0;
-    if (lane == 0) tile = atomicAdd(counter, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if ((uint64_t)tile >= tiles) return;
-    const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    if (x < p.width && y < row_end && !render_pixel<false, kNee, kWalk>(sc, p, y * p.width + x, out, nullptr))
+    unsigned unit = 0;
+    if (lane == 0) unit = atomicAdd(counter, 1u);
+    unit = __shfl_sync(0xffffffffu, unit, 0);
+    if ((uint64_t)unit >= units) return;
+    uint64_t x, y;
+    const bool in = unit_pixel(p, tiles_x, unit, x, y);
+    if (in && !render_pixel<false, kNee, kWalk>(sc, p, y * p.width + x, out, nullptr))
       render_pixel_f64(sc, p, y * p.width + x, out);
   }
 }
@@ -590,16 +606,16 @@ template <int BS, int kWalk>
 __global__ void __launch_bounds__(BS, 512 / BS) k_render_regen(const __grid_constant__ DevScene sc,
                                                              const __grid_constant__ RenderParams p, double* __restrict__ out,
                                                              unsigned int* __restrict__ counter) {
-  const uint64_t tiles_x = (p.width + 7) / 8, tiles = tiles_x * ((p.rows + 3) / 4);
-  const uint64_t row_end = p.row0 + p.rows;
+  const uint64_t tiles_x = (p.width + 7) / 8, units = work_units(p);
   const unsigned lane = threadIdx.x & 31;
   for (;;) {
-    unsigned tile = 0;
-    if (lane == 0) tile = atomicAdd(counter, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if ((uint64_t)tile >= tiles) return;
-    const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    render_pixel_regen<kWalk>(sc, p, x, y, x < p.width && y < row_end, out);
+    unsigned unit = 0;
+    if (lane == 0) unit = atomicAdd(counter, 1u);
+    unit = __shfl_sync(0xffffffffu, unit, 0);
+    if ((uint64_t)unit >= units) return;
+    uint64_t x, y;
+    const bool in = unit_pixel(p, tiles_x, unit, x, y);
+    render_pixel_regen<kWalk>(sc, p, x, y, in, out);
   }
 }
 
@@ -1016,19 +1032,55 @@ static unsigned persistent_grid(K kernel, int block, uint64_t work_items, size_t
 enum MegaVariant { kMegaNested = 0, kMegaRegen = 1 };
 constexpr double kRegenMeanPath = 3.0;
 
+/* Parts per tile (log2) of a render with few pixels.  A warp renders its
+ * tile's pixels as long as the longest of their paths takes at every bounce,
+ * so a part of the tile is done sooner than the whole; where the tiles do not
+ * fill the GPU the other parts run beside it.  Every tile is split as long
+ * as the parts fit the `room` warps the instance keeps resident (twice that
+ * for scenes of 4096 and more primitives, whose walks differ more from lane
+ * to lane, so that splitting pays beyond one full load).  The regeneration
+ * instance keeps all lanes busy and slows down as warps are added: 3/8 of its
+ * room.  Measured, whole tiles against this rule (the best split in brackets
+ * where it is another):
+ *   250k-triangle terrain 160x90x16 5.9 -> 2.1 ms, 320x180x16 6.7 -> 4.0,
+ *   480x270x8 3.7 -> 3.0 [2.9], 640x360x16 8.2 -> 8.2 [7.5]; 961x541x16 10.9
+ *   whole, 12.6 in halves;
+ *   17,000 spheres 160x90x16 3.3 -> 1.9 ms, 320x180x16 3.7 -> 3.2;
+ *   320 spheres 160x90x1 100 -> 87 us [81], 320x180x16 0.83 -> 0.85 ms;
+ *   Cornell box (regeneration) 64x48x64 4.9 -> 3.4 ms; 128x128x64 5.0 whole,
+ *   5.4 in halves. */
+static uint32_t choose_split(const RenderParams& p, uint64_t room) {
+  RenderParams q = p;
+  while (q.split < 4) {
+    q.split += 1;
+    if (work_units(q) > room) return q.split - 1;
+  }
+  return q.split;
+}
+
+/* Of the kernels with path regeneration (512 threads per SM). */
+static uint64_t regen_room() { return (uint64_t)sm_count() * (512 / 32) * 3 / 8; }
+
 template <int BS, int kWalk>
-static void launch_mega_bsf(const DevScene& v, const RenderParams& p, double* d_out, unsigned int* counter,
+static void launch_mega_bsf(const DevScene& v, const RenderParams& params, double* d_out, unsigned int* counter,
                             MegaVariant variant, cudaStream_t stream) {
-  const uint64_t npix = p.width * p.rows;
-  if (variant == kMegaRegen)
-    k_render_regen<BS, kWalk><<<persistent_grid(k_render_regen<BS, kWalk>, BS, npix), BS, 0, stream>>>(v, p, d_out,
-                                                                                                      counter);
-  else if (p.use_nee)
-    k_render_mega<BS, true, kWalk><<<persistent_grid(k_render_mega<BS, true, kWalk>, BS, npix), BS, 0, stream>>>(
+  RenderParams p = params;
+  const uint64_t sms = (uint64_t)sm_count() * (v.n_prims >= 4096 ? 2 : 1);
+  if (variant == kMegaRegen) {
+    p.split = choose_split(p, regen_room());
+    k_render_regen<BS, kWalk><<<persistent_grid(k_render_regen<BS, kWalk>, BS, work_units(p) * 32), BS, 0, stream>>>(
         v, p, d_out, counter);
-  else
-    k_render_mega<BS, false, kWalk><<<persistent_grid(k_render_mega<BS, false, kWalk>, BS, npix), BS, 0, stream>>>(
-        v, p, d_out, counter);
+  } else if (p.use_nee) {
+    p.split = choose_split(p, sms * mega_threads_per_sm(true, kWalk) / 32);
+    k_render_mega<BS, true, kWalk>
+        <<<persistent_grid(k_render_mega<BS, true, kWalk>, BS, work_units(p) * 32), BS, 0, stream>>>(v, p, d_out,
+                                                                                                  counter);
+  } else {
+    p.split = choose_split(p, sms * mega_threads_per_sm(false, kWalk) / 32);
+    k_render_mega<BS, false, kWalk>
+        <<<persistent_grid(k_render_mega<BS, false, kWalk>, BS, work_units(p) * 32), BS, 0, stream>>>(v, p, d_out,
+                                                                                                   counter);
+  }
 }
 
 template <int BS>
@@ -1588,16 +1640,15 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_forward_diff(const __grid_cons
                                                              const double* __restrict__ theta,
                                                              double* __restrict__ out, double* __restrict__ sample_L,
                                                              unsigned int* __restrict__ counter) {
-  const uint64_t tiles_x = (p.width + 7) / 8, tiles = tiles_x * ((p.rows + 3) / 4);
-  const uint64_t row_end = p.row0 + p.rows;
+  const uint64_t tiles_x = (p.width + 7) / 8, units = work_units(p);
   const unsigned lane = threadIdx.x & 31;
   for (;;) {
-    unsigned tile = 0;
-    if (lane == 0) tile = atomicAdd(counter, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if ((uint64_t)tile >= tiles) return;
-    const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    const bool valid = x < p.width && y < row_end;
+    unsigned unit = 0;
+    if (lane == 0) unit = atomicAdd(counter, 1u);
+    unit = __shfl_sync(0xffffffffu, unit, 0);
+    if ((uint64_t)unit >= units) return;
+    uint64_t x, y;
+    const bool valid = unit_pixel(p, tiles_x, unit, x, y);
     const uint64_t pix = y * p.width + x;
     Rng rng = rng_for_stream(p.seed, valid ? pix : 0);
     dv3 sum = V(0, 0, 0);
@@ -1660,17 +1711,16 @@ __global__ void __launch_bounds__(BS, (kCached ? 512 : 640) / BS) k_backward_dif
                                                               const double* __restrict__ sample_L,
                                                               unsigned int* __restrict__ counter) {
   double* g = grad + (size_t)((blockIdx.x * (BS / 32) + threadIdx.x / 32) % n_slices) * n_params;
-  const uint64_t tiles_x = (p.width + 7) / 8, tiles = tiles_x * ((p.rows + 3) / 4);
-  const uint64_t row_end = p.row0 + p.rows;
+  const uint64_t tiles_x = (p.width + 7) / 8, units = work_units(p);
   const unsigned lane = threadIdx.x & 31;
   const double inv_spp = 1.0 / (double)p.spp;
   for (;;) {
-    unsigned tile = 0;
-    if (lane == 0) tile = atomicAdd(counter, 1u);
-    tile = __shfl_sync(0xffffffffu, tile, 0);
-    if ((uint64_t)tile >= tiles) return;
-    const uint64_t x = (tile % tiles_x) * 8 + (lane & 7), y = p.row0 + (tile / tiles_x) * 4 + (lane >> 3);
-    const bool valid = x < p.width && y < row_end;
+    unsigned unit = 0;
+    if (lane == 0) unit = atomicAdd(counter, 1u);
+    unit = __shfl_sync(0xffffffffu, unit, 0);
+    if ((uint64_t)unit >= units) return;
+    uint64_t x, y;
+    const bool valid = unit_pixel(p, tiles_x, unit, x, y);
     const uint64_t pix = y * p.width + x;
     /* dL/dpixel of the band (rows row0 ..), pixel = sum * (1/spp), render.zig:144 */
     const dv3 adj = valid ? vscale(L3(dimg + 3 * (pix - p.row0 * p.width)), inv_spp) : V(0, 0, 0);
@@ -1779,6 +1829,7 @@ zt_status zt_forward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin, 
   RenderParams p = make_params(s, o);
   p.row0 = row_begin;
   p.rows = row_end - row_begin;
+  p.split = choose_split(p, regen_room());
   const size_t bytes = (size_t)(p.rows * o->width * 3) * sizeof(double);
   zt_diff_cache& cache = s->device->diff;
   cache.valid = false;
@@ -1810,7 +1861,7 @@ zt_status zt_forward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin, 
   }
   cudaError_t e = cudaMemsetAsync(s->device->counter, 0, sizeof(unsigned int), 0);
   if (e == cudaSuccess) {
-    k_forward_diff<128><<<persistent_grid(k_forward_diff<128>, 128, p.width * p.rows), 128>>>(
+    k_forward_diff<128><<<persistent_grid(k_forward_diff<128>, 128, work_units(p) * 32), 128>>>(
         launch_view(s), p, d_theta, d_out, cache.L, s->device->counter);
     e = cudaGetLastError();
   }
@@ -1861,6 +1912,7 @@ zt_status zt_backward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin,
   RenderParams p = make_params(s, o);
   p.row0 = row_begin;
   p.rows = row_end - row_begin;
+  p.split = choose_split(p, regen_room());
   const uint32_t n_params = (uint32_t)(s->materials.size() * 3);
   memset(d_colors, 0, n_params * sizeof(double));
   if (p.max_depth == 0 || n_params == 0) return ZT_OK;
@@ -1890,10 +1942,10 @@ zt_status zt_backward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin,
   if (e == cudaSuccess) e = cudaMemsetAsync(s->device->counter, 0, sizeof(unsigned int), 0);
   if (e == cudaSuccess) {
     if (sample_L)
-      k_backward_diff<128, true><<<persistent_grid(k_backward_diff<128, true>, 128, p.width * p.rows), 128>>>(
+      k_backward_diff<128, true><<<persistent_grid(k_backward_diff<128, true>, 128, work_units(p) * 32), 128>>>(
           launch_view(s), p, d_theta, d_img, d_grad, n_params, n_slices, sample_L, s->device->counter);
     else
-      k_backward_diff<128, false><<<persistent_grid(k_backward_diff<128, false>, 128, p.width * p.rows), 128>>>(
+      k_backward_diff<128, false><<<persistent_grid(k_backward_diff<128, false>, 128, work_units(p) * 32), 128>>>(
           launch_view(s), p, d_theta, d_img, d_grad, n_params, n_slices, nullptr, s->device->counter);
     k_sum_slices<<<(n_params + 127) / 128, 128>>>(d_grad, n_params, n_slices, d_grad + (size_t)n_slices * n_params);
     e = cudaGetLastError();

@@ -145,7 +145,7 @@ struct RenderParams {
   uint64_t width, height, spp, max_depth, seed;
   uint64_t row0, rows; /* the band of image rows rendered; output row 0 is image row row0 */
   uint32_t use_nee;  /* light_sampling && !lights.isEmpty() */
-  uint32_t pad;
+  uint32_t split;    /* log2 of the parts every 8x4 pixel tile is rendered in (render.cu, choose_split) */
 };
 
 }  // namespace zt
