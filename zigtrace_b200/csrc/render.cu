@@ -474,20 +474,16 @@ __host__ __device__ __forceinline__ uint64_t work_units(const RenderParams& p) {
  * by reference, and without it every thread would copy them to its stack. */
 constexpr int kMegaThreadsPerSm = 1024;
 constexpr int kMegaThreadsPerSmNoNee = 896;
-#ifndef ZT_FAST_THREADS_PER_SM
-#define ZT_FAST_THREADS_PER_SM 1024
-#endif
-#ifndef ZT_FAST_THREADS_PER_SM_NONEE
-#define ZT_FAST_THREADS_PER_SM_NONEE 1024
-#endif
 /* Resident threads per SM each megakernel and batch instance is built for
  * (__launch_bounds__): sets the register budget, 65,536 / threads.  The
- * fast-walk instances measured fastest at 1024 (64 registers): on the
- * 1M-triangle terrain 1026 Msamples/s against 992 at 896 and 933 at 768; on
- * the sphere-field batch 64.4 ms against 67.9 at 896 and 71.7 at 1280. */
+ * float-walk instances measured fastest at 1024 (64 registers): 1M-triangle
+ * terrain (16 spp) 31.1 ms against 31.2 at 896, 33.4 at 768 and 31.7 at
+ * 1152; the sphere-field batch 51.7 against 51.6, 52.7 and 57.0.  The
+ * checked walk without light sampling is built for 896: random spheres 3.98
+ * against 4.07 ms. */
 __host__ __device__ constexpr int mega_threads_per_sm(bool nee, int walk) {
-  return walk != kWalkF64 ? (nee ? ZT_FAST_THREADS_PER_SM : ZT_FAST_THREADS_PER_SM_NONEE)
-                          : (nee ? kMegaThreadsPerSm : kMegaThreadsPerSmNoNee);
+  return walk == kWalkF64 ? (nee ? kMegaThreadsPerSm : kMegaThreadsPerSmNoNee)
+                          : (walk == kWalkFloatChecked && !nee ? 896 : 1024);
 }
 
 template <int BS, bool kNee, int kWalk>
