@@ -94,3 +94,16 @@ def test_png_sizes_and_alignment(w, h, offset):
     got = out.cpu().numpy()
     assert (got[offset[1]:offset[1] + len(want)] == want).all()
     assert (got[:offset[1]] == 77).all() and (got[offset[1] + len(want):] == 77).all()
+
+
+def test_png_of_more_slices_than_two_digits_count():
+    """Above 64 x 64 slices of 8 KB the checksum's powers take a third digit."""
+    import torch
+    w, h = 6001, 2000
+    rgb = np.random.default_rng(7).integers(0, 256, 3 * w * h).astype(np.uint8)
+    want = np.frombuffer(zt.encode_png(rgb, w, h), np.uint8)
+    assert len(want) > 64 * 64 * 8192
+    d = torch.from_numpy(rgb).cuda()
+    out = torch.empty(len(want), dtype=torch.uint8, device="cuda")
+    zt.encode_png_device(d.data_ptr(), w, h, out.data_ptr(), len(want))
+    assert (out.cpu().numpy() == want).all()
