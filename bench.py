@@ -37,23 +37,26 @@ NOMINAL_SM_MHZ = 1965.0
 # workload, --clock-control none) and scaled by samples per launch: traffic
 # grows with the samples traced.  Keyed by (workload, precision); workloads
 # without a capture report null.
-NCU_DRAM_BYTES_PER_SAMPLE = {("triangle_heavy", "exact"): 2.527835e9 / (1920 * 1080 * 8),
-                             ("triangle_heavy", "fast"): (1.308102e9 + 1.654117e9) / (1920 * 1080 * 8)}
+NCU_DRAM_BYTES_PER_SAMPLE = {("triangle_heavy", "exact"): (0.944641e9 + 1.011825e9) / (1920 * 1080 * 8),
+                             ("triangle_heavy", "fast"): (0.993070e9 + 1.097135e9) / (1920 * 1080 * 8)}
 # What bounds the kernel instead of a pipe peak, from the same capture:
 # issue slots used, lanes active per warp instruction, FP64 pipe activity.
-NCU_EXECUTION = {("triangle_heavy", "exact"): {"issue_active_pct": 62.7, "lanes_per_warp_instruction": 8.27,
-                                               "fp64_pipe_active_pct": 45.9, "l1_hit_pct": 72.2, "l2_hit_pct": 84.3},
-                 ("triangle_heavy", "fast"): {"issue_active_pct": 59.5, "lanes_per_warp_instruction": 7.19,
-                                              "fp64_pipe_active_pct": 31.5, "fma_pipe_active_pct": 8.7,
-                                              "l1_hit_pct": 75.9, "l2_hit_pct": 83.1,
-                                              "top_stall": "long_scoreboard 5.4 cycles per issue"},
-                 ("batch", "exact"): {"issue_active_pct": 70.2, "lanes_per_warp_instruction": 14.23,
-                                      "fp64_pipe_active_pct": 44.5, "l1_hit_pct": 82.9, "l2_hit_pct": 88.5},
-                 ("batch", "fast"): {"issue_active_pct": 72.9, "lanes_per_warp_instruction": 14.32,
-                                     "fp64_pipe_active_pct": 25.6, "fma_pipe_active_pct": 16.0, "l1_hit_pct": 78.7,
-                                     "l2_hit_pct": 88.9, "top_stall": "long_scoreboard 2.9 cycles per issue"}}
+NCU_EXECUTION = {("triangle_heavy", "exact"): {"issue_active_pct": 59.7, "lanes_per_warp_instruction": 7.58,
+                                               "fp64_pipe_active_pct": 26.9, "fma_pipe_active_pct": 10.1,
+                                               "l1_hit_pct": 79.3, "l2_hit_pct": 84.7,
+                                               "top_stall": "long_scoreboard 5.3 cycles per issue"},
+                 ("triangle_heavy", "fast"): {"issue_active_pct": 60.2, "lanes_per_warp_instruction": 7.59,
+                                              "fp64_pipe_active_pct": 27.4, "fma_pipe_active_pct": 10.1,
+                                              "l1_hit_pct": 78.6, "l2_hit_pct": 84.3,
+                                              "top_stall": "long_scoreboard 5.3 cycles per issue"},
+                 ("batch", "exact"): {"issue_active_pct": 71.6, "lanes_per_warp_instruction": 14.10,
+                                      "fp64_pipe_active_pct": 24.8, "fma_pipe_active_pct": 16.9, "l1_hit_pct": 84.8,
+                                      "l2_hit_pct": 88.5, "top_stall": "wait 2.9 cycles per issue"},
+                 ("batch", "fast"): {"issue_active_pct": 75.4, "lanes_per_warp_instruction": 14.36,
+                                     "fp64_pipe_active_pct": 26.1, "fma_pipe_active_pct": 16.6, "l1_hit_pct": 81.3,
+                                     "l2_hit_pct": 88.6, "top_stall": "wait 2.9 cycles per issue"}}
 # The batched launch, captured whole (rank 0's batch, one launch), by precision.
-NCU_DRAM_BYTES_BATCH = {"exact": 0.160607e9 + 1.138117e9, "fast": 0.167182e9 + 2.485141e9}
+NCU_DRAM_BYTES_BATCH = {"exact": 0.095720e9 + 0.987772e9, "fast": 0.129497e9 + 1.905857e9}
 
 
 FP32_LANES_PER_SM = 128

@@ -145,7 +145,9 @@ zt_status zt_scene_build(zt_scene* scene);
  * without area) or hold non-finite coordinates are built on the host, as are
  * all scenes when no CUDA device (or too little device memory) is available;
  * *used_device (may be NULL) is 1 when the device built the BVH.
- * *build_ms (may be NULL) is the device time of the build. */
+ * *build_ms (may be NULL) is the device time of the build.  The shapes and
+ * the tree stay on the device (about 200 bytes a shape) until the scene is
+ * uploaded, changed or released. */
 zt_status zt_scene_build_device(zt_scene* scene, uint32_t* used_device, double* build_ms);
 
 /* Scene.build with the BVH the caller already built: the reference's

@@ -933,7 +933,8 @@ zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_no
   if (rc != ZT_OK) return rc;
   uint32_t got[2] = {0, 0};
   cudaError_t e = cudaMemsetAsync(flags, 0, sizeof got, 0);
-  if (e == cudaSuccess && n_prims) k_flat_prims<<<(n_prims + 255) / 256, 256>>>(t.shapes, t.indices, n_prims, prims, ids, flags);
+  if (e == cudaSuccess && n_prims)
+    k_flat_prims<<<(n_prims + 255) / 256, 256>>>(t.shapes, t.indices, n_prims, prims, ids, flags);
   const uint32_t n_pairs = n_nodes / 2;
   if (e == cudaSuccess && n_pairs)
     k_flat_pairs<<<(n_pairs + 255) / 256, 256>>>(t.nodes, n_pairs, eps[0], eps[1], eps[2], pairs, fpairs, flags);
@@ -986,7 +987,8 @@ zt_status device_build_bvh(zt_scene* s, double* build_ms) {
   const size_t o_lnodes = off; off += up(2 * n * sizeof(LNode));
   unsigned char *mem = nullptr, *kept = nullptr;
   if (pool_alloc((void**)&kept, k_bytes, 0, "device BVH build") != ZT_OK ||
-      pool_alloc((void**)&mem, off, 0, "device BVH build") != ZT_OK) { /* no device, or not enough device memory: the host builds it */
+      pool_alloc((void**)&mem, off, 0, "device BVH build") != ZT_OK) {
+    /* no device, or not enough device memory: the host builds it */
     if (kept) cudaFreeAsync(kept, 0);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);

@@ -488,7 +488,8 @@ __host__ __device__ constexpr int mega_threads_per_sm(bool nee, int walk) {
 
 template <int BS, bool kNee, int kWalk>
 __global__ void __launch_bounds__(BS, mega_threads_per_sm(kNee, kWalk) / BS)
-    k_render_mega(const __grid_constant__ DevScene sc, const __grid_constant__ RenderParams p, double* __restrict__ out, unsigned int* __restrict__ counter) {
+    k_render_mega(const __grid_constant__ DevScene sc, const __grid_constant__ RenderParams p,
+                  double* __restrict__ out, unsigned int* __restrict__ counter) {
   const uint64_t tiles_x = (p.width + 7) / 8, units = work_units(p);
   const unsigned lane = threadIdx.x & 31;
   for (;;) {
@@ -553,7 +554,8 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
         const DMat& mat = sc.mats[hit.material];
         const dv3 le = (mat.kind == kEmissive && hit.front_face) ? L3(mat.color) : V(0, 0, 0);
         if (vmaxc(le) > 0) {
-          const double wt = prev_pdf > 0 ? power_weight(prev_pdf, lights_pdf_hit<kWalk != kWalkF64>(sc, ro, hit.point)) : 1.0;
+          const double wt =
+              prev_pdf > 0 ? power_weight(prev_pdf, lights_pdf_hit<kWalk != kWalkF64>(sc, ro, hit.point)) : 1.0;
           radiance = radiance + vscale(vmul(throughput, le), wt);
         }
         if (mat.kind == kLambertian && use_nee)
