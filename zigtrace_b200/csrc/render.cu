@@ -419,7 +419,8 @@ __device__ __forceinline__ bool render_pixel(const DevScene& sc, const RenderPar
   Rng rng = rng_for_stream(p.seed, y * p.width + x);
   dv3 sum = V(0, 0, 0);
   bool unsure = false;
-  for (uint64_t i = 0; i < p.spp; ++i) {
+  typedef typename Counter<kWalk>::type Count;
+  for (Count i = 0; i < (Count)p.spp; ++i) {
     const double s = ((double)x + rng_float(rng)) / w;
     const double t = ((double)y + rng_float(rng)) / h;
     dv3 ro, rd;
@@ -1102,6 +1103,7 @@ static bool valid_block_size(uint32_t bs) { return bs == 0 || bs == 64 || bs == 
 constexpr uint32_t kFastMinPrimitives = 64;
 static Walk choose_walk(const zt_scene* s, const RenderParams& p, uint32_t precision, bool small_scenes_f64 = true) {
   if (!s->device || !s->device->view.fast_ok) return kWalkF64;
+  if (p.spp > 0xFFFFFFFFull || p.max_depth > 0xFFFFFFFFull) return kWalkF64; /* 32-bit counters */
   if (precision != ZT_PRECISION_FAST && !s->device->view.verify_ok) return kWalkF64;
   if (small_scenes_f64 && s->device->view.n_prims < kFastMinPrimitives) return kWalkF64;
   const double* o = p.cam.origin;
