@@ -603,6 +603,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock, 8) k_small(Subtree* __res
        * axis has the same two sides and the same cost: the first axis and
        * bin 0 are findSplit's choice. */
       const uint32_t e0 = idx[en.first], e1 = idx[en.first + c - 1];
+      __syncwarp(); /* every lane has its two before lane 0 may exchange them below */
       const DBox b0 = boxes[e0], b1 = boxes[e1];
       LNode rec;
       rec.bounds = b0;
