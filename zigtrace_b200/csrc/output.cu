@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "output.cuh"
+#include "png_crc.h"
 #include "scene_host.h"
 
 namespace zt {
@@ -179,23 +180,6 @@ zt_status launch_encode_rgb8(const double* d_px, uint64_t n_values, uint32_t ton
 }
 
 /* ---------------------------------------------------------------- CRC ---- */
-/* CRC-32 of PNG (ISO-HDLC: reflected polynomial 0xEDB88320, register
- * preset to all ones, result complemented).  Polynomials over GF(2) are
- * held bit-reflected: bit 31 is the coefficient of x^0. */
-constexpr uint32_t kCrcPoly = 0xEDB88320u;
-
-/* a * b mod P. */
-__host__ __device__ constexpr uint32_t crc_mulmod(uint32_t a, uint32_t b) {
-  uint32_t p = 0;
-  for (int i = 0; i < 32; ++i) {
-    p ^= b & (0u - (a >> 31));
-    a <<= 1;
-    b = (b >> 1) ^ (kCrcPoly & (0u - (b & 1u))); /* b *= x */
-  }
-  return p;
-}
-constexpr uint32_t kCrcOne = 1u << 31; /* x^0 */
-
 /* x^n mod P; x has order 2^32 - 1, so x^-n is x^(2^32 - 1 - n). */
 struct CrcSquares {
   uint32_t v[64]; /* x^(2^k) */
@@ -217,12 +201,6 @@ static uint32_t crc_xpow(uint64_t n) {
   return r;
 }
 
-/* Register update for one input byte. */
-__host__ __device__ constexpr uint32_t crc_byte(uint32_t i) {
-  uint32_t c = i;
-  for (int k = 0; k < 8; ++k) c = (c >> 1) ^ (kCrcPoly & (0u - (c & 1u)));
-  return c;
-}
 struct CrcTable {
   uint32_t byte[256];
 };
@@ -232,44 +210,6 @@ static CrcTable make_crc_table() {
   return T;
 }
 
-constexpr int kPngThreads = 256;
-constexpr uint32_t kPngSeg = 32;                       /* bytes per thread */
-constexpr uint32_t kPngSlice = kPngThreads * kPngSeg;  /* 8 KB per block */
-
-/* Powers of x: seg[t] = x^(8 * kPngSeg * (kPngThreads - 1 - t)), what follows
- * a thread's segment in its slice; slice[d][k] = x^(8 * kPngSlice * k *
- * 64^d), the digits base 64 of the number of slices that follow. */
-struct CrcPowers {
-  uint32_t seg[kPngThreads];
-  uint32_t slice[3][64];
-  uint32_t tab[256][4]; /* tab[i][j]: register update of byte i followed by j zero bytes */
-};
-constexpr CrcPowers make_crc_powers() {
-  CrcPowers P{};
-  uint32_t x = kCrcOne >> 1; /* x^1 */
-  for (uint32_t n = 1; n < 8 * kPngSeg; n <<= 1) x = crc_mulmod(x, x);
-  uint32_t r = kCrcOne;
-  for (int t = kPngThreads - 1; t >= 0; --t) {
-    P.seg[t] = r;
-    r = crc_mulmod(r, x);
-  }
-  for (int d = 0; d < 3; ++d) { /* r = x^(8 * kPngSlice * 64^d) */
-    uint32_t q = kCrcOne;
-    for (int k = 0; k < 64; ++k) {
-      P.slice[d][k] = q;
-      q = crc_mulmod(q, r);
-    }
-    r = q;
-  }
-  for (uint32_t i = 0; i < 256; ++i) {
-    uint32_t c = i;
-    for (int j = 0; j < 4; ++j) {
-      c = j == 0 ? crc_byte(c) : (c >> 8) ^ crc_byte(c & 255u);
-      P.tab[i][j] = c;
-    }
-  }
-  return P;
-}
 static __device__ __align__(16) const CrcPowers c_crc_powers = make_crc_powers();
 
 static uint32_t crc32_host(const uint8_t* p, size_t n, const CrcTable& T, uint32_t c = 0xFFFFFFFFu) {
@@ -520,9 +460,9 @@ __global__ void __launch_bounds__(kPngThreads) k_png_slices(const uint8_t* __res
   }
   __syncthreads();
   if (t == 0) {
-    uint32_t n = gridDim.x - 1 - blockIdx.x;
-    uint32_t follow = c_crc_powers.slice[0][n & 63u]; /* x^(8 * bytes of the slices that follow) */
-    for (int d = 1; d < 3 && (n >>= 6) != 0; ++d) follow = crc_mulmod_tab(tab, follow, c_crc_powers.slice[d][n & 63u]);
+    const uint32_t follow = crc_slices_power(c_crc_powers, gridDim.x - 1 - blockIdx.x, [&](uint32_t a, uint32_t b) {
+      return crc_mulmod_tab(tab, a, b);
+    });
     uint32_t s0 = 0, s1 = 0, s2 = 0;
     for (int k = 0; k < kPngThreads / 32; ++k) {
       s0 += part[0][k];
