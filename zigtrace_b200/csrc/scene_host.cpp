@@ -517,8 +517,9 @@ static float f32_up(double x) {
 }
 
 /* The fast traversal's float records (zt_types.h FPair): every box of the
- * f64 tree moved outward by eps[axis] = 2^-20 * M[axis], M the largest
- * |bound| of the root box on that axis, then rounded outward.  The margin
+ * f64 tree moved outward by eps[axis] = 2^-20 * M[axis] (kFastMinMargin at
+ * least), M the largest |bound| of the root box on that axis, then rounded
+ * outward.  The margin
  * covers the float slab test's rounding of box coordinates (the error
  * analysis is in zt_fast.cuh), so a ray whose f64 slab test reaches a box
  * also reaches its float copy.  Left empty (fast traversal unavailable) when
@@ -534,7 +535,7 @@ static void make_fast_records(const zt_scene* s, FlatScene* f, bool with_tree) {
   for (int k = 0; k < 3; ++k) {
     const double m = std::max(std::fabs(s->nodes[0].bmin[k]), std::fabs(s->nodes[0].bmax[k]));
     if (!(m <= kFastMaxCoord)) return; /* also rejects NaN */
-    eps[k] = std::ldexp(m, -20);
+    eps[k] = std::max(std::ldexp(m, -20), kFastMinMargin);
   }
   if (with_tree)
     for (const HostNode& nd : s->nodes)

@@ -22,7 +22,7 @@
  *    reciprocal's 2^-23);
  *  - the |c| part is covered by the records: every bound is moved outward by
  *    eps = 2^-20 M (M the largest |bound| on that axis; 4x the 2 2^-23 M
- *    needed), which moves a near plane's distance down and a far plane's up
+ *    needed; kFastMinMargin at least), which moves a near plane's distance down and a far plane's up
  *    by eps / |d|;
  *  - the |o| part is covered per ray: w = 2^-20 |n| (2.3x the 3.5 2^-23 |o I|
  *    needed) is subtracted from near planes and added to far planes;
@@ -32,8 +32,19 @@
  *    rounding (2^-53 relative) is far inside these margins.
  *  - A zero or tiny direction component has its reciprocal clamped to +-K
  *    with K |o| <= 1e37 and K M <= 1e37 (M <= kFastMaxCoord), so no product
- *    overflows; the plane distances then keep their signs (the ray is inside
- *    or outside that slab), which is all the test uses on that axis.
+ *    overflows.  Near distances only get smaller by that (in magnitude where
+ *    the ray starts outside the slab, in sign where it starts inside).  The
+ *    far distance does too, and must still exceed every distance t at which
+ *    the ray can be in the slab: it is at least 3/4 K eps - t (eps the
+ *    record's margin, of which the roundings above take at most a quarter;
+ *    a component below 1/K moves the ray by at most t/K on the axis), so
+ *    3/4 K eps >= 2 t is needed.  The scene's bounds end at t <= 1.8 (|o| +
+ *    1.8 M) / |d|, |d| >= 0.28 (fray_make).  For |o| <= 1e7 that is 2e8, and
+ *    3/4 K eps >= 7e14 (K = 1e30, eps >= kFastMinMargin).  Beyond, K = 1e37 /
+ *    |o| falls as t rises: at kFastMaxOrigin = 1e10, t <= 6.5e10 and 3/4 K eps
+ *    >= 7e11.  (At the 1e30 this limit once was, a box straight ahead of a
+ *    ray parallel to an axis was missed from about 3e18 on, and from less in
+ *    flat scenes.)
  * Entry distances are lower bounds of the exact ones, so `entry.t > closest`
  * pruning against closest rounded up never drops a node the reference
  * visits, and leaves are tested with the reference's f64 primitive tests.
@@ -109,10 +120,10 @@ ZT_D float fmin3f(float a, float b, float c) {
   return r;
 }
 
-/* Largest |origin| (component sum) the float test takes.  Rays from farther
- * away (a hit far out on an unbounded plane), with a NaN, or with a direction
- * far from unit length make the pixel unsure. */
-constexpr float kFastMaxOrigin = 1e30f;
+/* Largest |origin| (component sum) the float test takes (derived above).
+ * Rays from farther away (a hit far out on an unbounded plane), with a NaN, or
+ * with a direction far from unit length make the pixel unsure. */
+constexpr float kFastMaxOrigin = 1e10f;
 
 ZT_D bool fray_make(dv3 o, dv3 d, FRay& r) {
   const float o3[3] = {(float)o.x, (float)o.y, (float)o.z};
@@ -120,7 +131,7 @@ ZT_D bool fray_make(dv3 o, dv3 d, FRay& r) {
   const float om = fmaxf(fabsf(o3[0]), fmaxf(fabsf(o3[1]), fabsf(o3[2])));
   const float os = fabsf(o3[0]) + fabsf(o3[1]) + fabsf(o3[2]); /* sums: a NaN component fails the test */
   const float ds = fabsf(d3[0]) + fabsf(d3[1]) + fabsf(d3[2]);
-  if (!(os <= kFastMaxOrigin && ds >= 1e-6f && ds <= 1e6f)) return false;
+  if (!(os <= kFastMaxOrigin && ds >= 0.5f && ds <= 2.0f)) return false; /* ds: 1 to sqrt(3) of a unit vector */
   const float K = om > 1e7f ? 1e37f / om : 1e30f; /* K |o| <= 1e37, K * kFastMaxCoord <= 1e37 */
 #pragma unroll
   for (int a = 0; a < 3; ++a) {

@@ -72,6 +72,10 @@ constexpr uint32_t kFastMaxLeaf = (1u << (32 - kFastCountShift)) - 1;
 /* Largest |coordinate| (of the scene's bounds and of ray origins) the float
  * slab test handles: products with the clamped reciprocal stay finite. */
 constexpr double kFastMaxCoord = 1e7;
+/* Least outward margin of a float box: what a clamped reciprocal leaves of a
+ * slab's far distance has to exceed every distance along the ray
+ * (zt_fast.cuh). */
+constexpr double kFastMinMargin = 1e-15;
 
 struct ZT_ALIGN(16) DMat {
   double color[3];
