@@ -127,8 +127,10 @@ zt_status pool_alloc(void** p, size_t bytes, cudaStream_t st, const char* what) 
   cudaMemPool_t pool = nullptr;
   zt_status rc = device_pool(&pool);
   if (rc != ZT_OK) return rc;
-  ZT_CUDA(cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 256, pool, st), what);
-  return ZT_OK;
+  const cudaError_t e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 256, pool, st);
+  if (e == cudaSuccess) return ZT_OK;
+  cudaGetLastError(); /* reported here; a caller that does without it must not meet it again at its next launch */
+  return cuda_fail(e, what);
 }
 
 static void pool_free(void* p, cudaStream_t st) {
@@ -351,6 +353,8 @@ static zt_status upload(zt_scene* s, bool sync = true) {
   zt_status rc = ZT_OK;
   if (!s->staging && !s->shapes.empty() && upload_flattened(s, dev) == ZT_OK)
     return s->pilot_valid ? ZT_OK : pilot_paths(s);
+  cudaGetLastError();     /* of the attempt above */
+  release_device_tree(s); /* its memory may be what the block below needs */
   rc = make_staging(s);
   if (rc != ZT_OK) return rc;
   const zt_host_staging* h = s->staging;
