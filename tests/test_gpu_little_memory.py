@@ -36,7 +36,7 @@ UPLOAD = COMMON + """
 device = {device}
 small = spheres(500, 0).build(device=device)   # kernels and their local memory are loaded
 zt.render(small, o)
-n = 500_000
+n = 2_200_000 if device else 500_000           # of this size the build leaves nothing but the tree in the pool
 scene = spheres(n, 1).build(device=device)
 assert scene.built_on_device == device
 block = scene.staging_bytes()
@@ -45,7 +45,7 @@ held = hold_all_but(block + beside // 2 if not device else block - beside // 2)
 img = zt.render(scene, o).pixels
 del held
 torch.cuda.empty_cache()
-assert img.tobytes() == zt.render(spheres(n, 1).build(), o).pixels.tobytes()
+assert img.tobytes() == zt.render(spheres(n, 1).build(device=device), o).pixels.tobytes()
 """
 
 
@@ -58,3 +58,20 @@ def run(program):
 def test_upload_with_room_for_the_block_only(device):
     """device=True: the tree that the device build left makes room for it."""
     run(UPLOAD.format(device=device))
+
+
+BUILD = COMMON + """
+small = spheres(500, 0).build(device=True)
+small.upload()
+n = 2_500_000
+scene = spheres(n, 1)
+free = torch.cuda.mem_get_info()[0]
+scene.build(device=True)
+taken = free - torch.cuda.mem_get_info()[0]
+assert scene.built_on_device
+assert taken <= 196 * n + (64 << 20), taken    # shapes, permutation and nodes, until the upload
+"""
+
+
+def test_a_large_device_build_gives_its_scratch_back():
+    run(BUILD)
