@@ -67,15 +67,19 @@
  *    primitive, and it is the least hit of a superset of what that walk
  *    tests.  No hit in the superset means none in the f64 walk.
  * Where either is in doubt `unsure` is set and the caller renders the pixel
- * again with the f64 walk (one pixel in some ten thousand: the flag costs a
- * register, where a call of the f64 walk from inside this one measured 7% on
+ * again with the f64 walk (none of the images measured below: the flag costs
+ * a register, where a call of the f64 walk from inside this one measured 7% on
  * the 1M-triangle terrain and 12% on the sphere fields).  Rays the float
- * test does not take (fray_make) go the same way.  The margins of
- * walk_reaches: the f64 slab test and o + t d err by at most
- * 2^-50 (M + |o|) on an axis (M the largest bound: three roundings of a
- * plane distance, two of the point), and 2^-46 (M + |o|) is asked; the
- * point's offset from the primitive and the primitive's extents are rounded
- * to float (2^-24 relative), and 2^-20 of the extent is asked.
+ * test does not take (fray_make) go the same way.  The margin walk_reaches
+ * asks for is derived in zt_reach.h.  It is compared in f64: in single
+ * precision the extents' rounding had to be allowed for (2^-20 of them), which
+ * left the middle of a ground made of a large sphere in doubt, 1.4 units
+ * around the pole at radius 1000: of random spheres on such a ground
+ * (1280x720x16) 2.7% of the pixels were rendered twice, and the image took
+ * 7.3 ms, now 3.85, with the f64 walk alone 5.6; at radius 5000, 55%, 12.0 ms,
+ * 3.87 and 5.6.  The f64
+ * comparisons also take less time than the conversions did (random spheres
+ * 3.78 -> 3.61 ms, terrain unchanged).
  * Measured, against the f64 walk with its 128-byte records: 250k-triangle
  * terrain 961x541x16 14.56 -> 11.14 ms, random spheres 1280x720x16 5.35 ->
  * 4.09 ms, 256 sphere fields 71.9 -> 54.8 ms.
@@ -85,6 +89,8 @@
  */
 #ifndef ZT_FAST_CUH
 #define ZT_FAST_CUH
+
+#include "zt_reach.h"
 
 namespace zt {
 
@@ -163,31 +169,11 @@ ZT_D bool fslab(unsigned long long bx, unsigned long long by, unsigned long long
 
 /* Whether the f64 walk is certain to reach the leaf of primitive p, hit at
  * `point` by a ray from o: the point is inside the primitive's box by the
- * margins derived above. */
+ * margin derived in zt_reach.h. */
 ZT_D bool walk_reaches(const DevScene& sc, const DPrim& p, dv3 o, dv3 point) {
+  const double m = kReachMargin * ((double)sc.freach + fabs(o.x) + fabs(o.y) + fabs(o.z));
   const dv3 h = point - L3(p.a);
-  const float q[3] = {(float)h.x, (float)h.y, (float)h.z};
-  const float slack = (sc.freach + fabsf((float)o.x) + fabsf((float)o.y) + fabsf((float)o.z)) * 0x1.0p-46f;
-  bool in = true;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    float lo, hi;
-    if (p.kind == kTriangle) {
-      const float e1 = (float)p.a[3 + a], e2 = (float)p.a[6 + a];
-      lo = fmin3f(e1, e2, 0.0f);
-      hi = fmax3f(e1, e2, 0.0f);
-      if (hi - lo < 0.99e-6f) { /* Aabb.pad adds 5e-7 on both sides, aabb.zig:30-39 */
-        lo -= 4.95e-7f;
-        hi += 4.95e-7f;
-      }
-    } else {
-      hi = fabsf((float)p.a[3]);
-      lo = -hi;
-    }
-    const float m = slack + fmaxf(-lo, hi) * 0x1.0p-20f;
-    in = in && q[a] >= lo + m && q[a] <= hi - m;
-  }
-  return in;
+  return reach_inside(p.kind == kTriangle, p.a, h.x, h.y, h.z, m);
 }
 
 /* One 64-byte record: both children's axis pairs and payload words. */
