@@ -58,7 +58,13 @@
  *
  * The checked walk (kVerify, ZT_PRECISION_EXACT) detects those two cases, so
  * its results are the f64 walk's bit for bit:
- *  - a tie: another primitive is hit at exactly the closest distance;
+ *  - a tie: another primitive is hit at exactly the closest distance.  In
+ *    one leaf both walks test the primitives in the same order and the first
+ *    keeps the hit; only a tie between leaves is in doubt.  (Coincident
+ *    primitives have one centroid, which no split separates.  With every tie
+ *    in doubt, the 250k-triangle terrain 961x541x16 with each triangle twice
+ *    took 21.0 ms, with each fiftieth twice 22.6; now 13.8 and 10.6, the f64
+ *    walk alone 17.3 and 14.0.)
  *  - a hit whose leaf the f64 walk might miss: walk_reaches shows that the
  *    hit point lies inside the primitive's box by more than the f64 test's
  *    rounding.  Every ancestor's box holds that box (boxes_nested), so the
@@ -76,10 +82,9 @@
  * left the middle of a ground made of a large sphere in doubt, 1.4 units
  * around the pole at radius 1000: of random spheres on such a ground
  * (1280x720x16) 2.7% of the pixels were rendered twice, and the image took
- * 7.3 ms, now 3.85, with the f64 walk alone 5.6; at radius 5000, 55%, 12.0 ms,
- * 3.87 and 5.6.  The f64
- * comparisons also take less time than the conversions did (random spheres
- * 3.78 -> 3.61 ms, terrain unchanged).
+ * 7.3 ms, now 3.85, with the f64 walk alone 5.6; at radius 5000 55%, 12.0 ms,
+ * 3.87 and 5.6.  The f64 comparisons also take less time than the conversions
+ * did (random spheres 3.78 -> 3.61 ms, terrain unchanged).
  * Measured, against the f64 walk with its 128-byte records: 250k-triangle
  * terrain 961x541x16 14.56 -> 11.14 ms, random spheres 1280x720x16 5.35 ->
  * 4.09 ms, 256 sphere fields 71.9 -> 54.8 ms.
@@ -239,18 +244,22 @@ ZT_D int32_t scene_query_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, dou
         if (et > cl32) continue; /* bvh.zig:97, against closest rounded up */
         const uint32_t cnt = w >> kFastCountShift, first = w & kFastFirstMask;
         if (cnt > 0) {
+          /* in a leaf a hit of its own is kept as -2 - k (with a flag beside it terrain 11.2 ms against 11.05) */
           for (uint32_t k = first; k < first + cnt; ++k) {
             double th;
             if (bounded_t<kVerify>(sc.prims[k], o, d, tmin, closest, th)) {
-              if (kVerify && !(th < closest)) { /* a tie: the f64 walk's visiting order decides */
-                unsure = true;
+              if (kVerify && !(th < closest)) {
+                /* a tie (or a NaN): in one leaf the first primitive keeps the hit, as in the f64 walk; between
+                 * leaves that walk's visiting order decides */
+                if (best_k >= -1 || !(th == closest)) unsure = true;
               } else {
                 closest = th;
-                best_k = (int32_t)k;
+                best_k = kVerify ? -2 - (int32_t)k : (int32_t)k;
                 cl32 = __double2float_ru(th);
               }
             }
           }
+          if (kVerify && best_k < -1) best_k = -2 - best_k;
           continue;
         }
         const FRec r = frec_load(sc.fpairs + first);
