@@ -259,7 +259,8 @@ static void set_view(zt_device_buffers* d, const zt_host_staging* h) {
  * time (released and uploaded again, frame after frame) then gets its pinned
  * image, read back from the device, so that later uploads are one copy.
  * Anything but ZT_OK: nothing is resident (make_staging is tried next; it
- * also serves scenes without bounded shapes). */
+ * also serves scenes without bounded shapes, and imported trees with leaves
+ * too large for the float records, which it leaves out). */
 static zt_status upload_flattened(zt_scene* s, int dev) {
   FlatScene f;
   zt_host_staging* h = new (std::nothrow) zt_host_staging();
@@ -311,8 +312,10 @@ static zt_status upload_flattened(zt_scene* s, int dev) {
       rc = flatten_on_device(t, (uint32_t)n, (uint32_t)nn, f.fast_eps, (DPrim*)(b + h->off_prims),
                              (int32_t*)(b + h->off_ids), (DPair*)(b + h->off_pairs),
                              f.view.fast_ok ? (FPair*)(b + h->off_fpairs) : nullptr, &max_leaf, &nan);
-    if (max_leaf > kFastMaxLeaf || s->nodes[0].count > kFastMaxLeaf) f.view.fast_ok = 0;
+    if (s->nodes[0].count > kFastMaxLeaf) f.view.fast_ok = 0;
     if (nan) f.view.verify_ok = 0;
+    if (rc == ZT_OK && f.view.fast_ok && max_leaf > kFastMaxLeaf) /* laid out with float records, which there are not */
+      rc = fail(ZT_ERR_INVALID_ARGUMENT, "a leaf too large for the float records: flattened on the host");
   }
   pool_free(copy, 0);
   if (rc == ZT_OK && e != cudaSuccess) rc = cuda_fail(e, "upload scene");
@@ -1366,7 +1369,9 @@ zt_status zt_scene_upload_bytes(zt_scene* s, uint64_t* bytes) {
       return fail(ZT_ERR_OUT_OF_MEMORY, "OutOfMemory while flattening the scene");
     }
     const size_t pairs = s->nodes.size() / 2;
-    layout(f, s->shapes.size(), pairs, f.view.fast_ok ? pairs : 0, &h);
+    bool fast = f.view.fast_ok;
+    for (const HostNode& nd : s->nodes) fast = fast && nd.count <= kFastMaxLeaf;
+    layout(f, s->shapes.size(), pairs, fast ? pairs : 0, &h);
     *bytes = h.bytes;
     return ZT_OK;
   }
