@@ -75,3 +75,36 @@ assert taken <= 196 * n + (64 << 20), taken    # shapes, permutation and nodes, 
 
 def test_a_large_device_build_gives_its_scratch_back():
     run(BUILD)
+
+
+GRADIENTS = COMMON + """
+def many_materials(n):
+    s = spheres(60, 3)
+    rng = np.random.default_rng(5)
+    m = np.concatenate([s.materials, np.tile(s.materials[:1], n)])
+    m["color"][4:] = rng.random((n, 3))
+    t = zt.Scene()
+    t.background, t.camera = s.background, s.camera
+    t.add_materials(m)
+    t.add_shapes(s.shapes)
+    return t
+
+g = np.ones((o.width * o.height, 3))
+few = many_materials(8).build()
+zt.forward(few, o)
+zt.backward(few, o, g)
+scene = many_materials(200_000).build()
+zt.forward(scene, o)
+held = hold_all_but(24 << 20)                  # a slice of gradients is 4.8 MB, all slices 64 MB
+got = zt.backward(scene, o, g)
+del held
+torch.cuda.empty_cache()
+want = zt.backward(scene, o, g)
+assert np.abs(want).max() > 1
+np.testing.assert_allclose(got, want, rtol=1e-11, atol=1e-11 * np.abs(want).max())
+"""
+
+
+def test_backward_with_room_for_few_gradient_slices():
+    """Sums of at most 64 x 48 x 2 x 6 terms in another order."""
+    run(GRADIENTS)

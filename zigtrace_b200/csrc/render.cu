@@ -1936,18 +1936,25 @@ zt_status zt_backward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin,
   double *d_theta = nullptr, *d_img = nullptr, *d_grad = nullptr;
   if ((rc = upload_theta(th, &d_theta)) != ZT_OK) return rc;
   rc = pool_alloc((void**)&d_img, img_bytes, 0, "allocate image adjoint");
-  /* a slice per resident warp (at most five blocks of four warps per SM), within 64 MiB */
-  const uint32_t n_slices = (uint32_t)std::max<uint64_t>(
+  /* a slice per resident warp (at most five blocks of four warps per SM), within 64 MiB; fewer, down to one,
+   * where the device has no room for them */
+  uint32_t n_slices = (uint32_t)std::max<uint64_t>(
       1, std::min<uint64_t>((uint64_t)sm_count() * 20, (64ull << 20) / (n_params * sizeof(double))));
-  const size_t grad_bytes = (size_t)n_slices * n_params * sizeof(double);
-  if (rc == ZT_OK) rc = pool_alloc((void**)&d_grad, grad_bytes + n_params * sizeof(double), 0, "allocate gradients");
+  size_t grads = 0; /* the slices; behind them their sum, which a single one is itself */
+  while (rc == ZT_OK) {
+    grads = (size_t)n_slices * n_params;
+    rc = pool_alloc((void**)&d_grad, (grads + (n_slices > 1 ? n_params : 0)) * sizeof(double), 0, "allocate gradients");
+    if (rc != ZT_ERR_OUT_OF_MEMORY || n_slices == 1) break;
+    n_slices = (n_slices + 7) / 8;
+    rc = ZT_OK;
+  }
   if (rc != ZT_OK) {
     pool_free(d_theta, 0);
     pool_free(d_img, 0);
     return rc;
   }
   cudaError_t e = cudaMemcpy(d_img, d_image, img_bytes, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d_grad, 0, grad_bytes, 0);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_grad, 0, grads * sizeof(double), 0);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->device->counter, 0, sizeof(unsigned int), 0);
   if (e == cudaSuccess) {
     if (sample_L)
@@ -1956,10 +1963,11 @@ zt_status zt_backward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin,
     else
       k_backward_diff<128, false><<<persistent_grid(k_backward_diff<128, false>, 128, work_units(p) * 32), 128>>>(
           launch_view(s), p, d_theta, d_img, d_grad, n_params, n_slices, nullptr, s->device->counter);
-    k_sum_slices<<<(n_params + 127) / 128, 128>>>(d_grad, n_params, n_slices, d_grad + (size_t)n_slices * n_params);
+    if (n_slices > 1) k_sum_slices<<<(n_params + 127) / 128, 128>>>(d_grad, n_params, n_slices, d_grad + grads);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(d_colors, d_grad + (size_t)n_slices * n_params, n_params * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(d_colors, d_grad + (n_slices > 1 ? grads : 0), n_params * sizeof(double), cudaMemcpyDeviceToHost);
   pool_free(d_theta, 0);
   pool_free(d_img, 0);
   pool_free(d_grad, 0);
