@@ -879,8 +879,9 @@ __global__ void __launch_bounds__(256) k_flat_prims(const zt_shape* __restrict__
 
 /* One thread per pair record r: reference nodes 2r+1 and 2r+2. */
 __global__ void __launch_bounds__(256) k_flat_pairs(const HostNode* __restrict__ nodes, uint32_t n_pairs, double ex,
-                                                    double ey, double ez, DPair* __restrict__ pairs,
-                                                    FPair* __restrict__ fpairs, uint32_t* __restrict__ flags) {
+                                                    double ey, double ez, bool ordered,
+                                                    DPair* __restrict__ pairs, FPair* __restrict__ fpairs,
+                                                    uint32_t* __restrict__ flags) {
   const uint32_t r = blockIdx.x * 256 + threadIdx.x;
   if (r >= n_pairs) return;
   const double eps[3] = {ex, ey, ez};
@@ -899,11 +900,18 @@ __global__ void __launch_bounds__(256) k_flat_pairs(const HostNode* __restrict__
     p.first[c] = nd.count > 0 ? nd.first : (nd.first - 1) / 2;
     p.count[c] = nd.count;
     f.word[c] = nd.count << kFastCountShift | p.first[c];
-    f.pad[c] = 0;
     if (nd.count > kFastMaxLeaf) atomicMax(flags, nd.count);
   }
   pairs[r] = p;
-  if (fpairs) fpairs[r] = f;
+  if (!fpairs) return;
+  f.split = kNoSplit;
+  f.pad = 0;
+  if (ordered) { /* the right child's first leaf */
+    uint32_t at = 2 * r + 2;
+    while (nodes[at].count == 0) at = nodes[at].first;
+    f.split = nodes[at].first;
+  }
+  fpairs[r] = f;
 }
 
 }  // namespace
@@ -927,8 +935,8 @@ bool device_tree(const zt_scene* s, DeviceTree* out) {
   return true;
 }
 
-zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_nodes, const double eps[3], DPrim* prims,
-                            int32_t* ids, DPair* pairs, FPair* fpairs, uint32_t* max_leaf, bool* nan) {
+zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_nodes, const double eps[3], bool ordered,
+                            DPrim* prims, int32_t* ids, DPair* pairs, FPair* fpairs, uint32_t* max_leaf, bool* nan) {
   uint32_t* flags = nullptr;
   zt_status rc = pool_alloc((void**)&flags, 2 * sizeof(uint32_t), 0, "flatten: flags");
   if (rc != ZT_OK) return rc;
@@ -938,7 +946,8 @@ zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_no
     k_flat_prims<<<(n_prims + 255) / 256, 256>>>(t.shapes, t.indices, n_prims, prims, ids, flags);
   const uint32_t n_pairs = n_nodes / 2;
   if (e == cudaSuccess && n_pairs)
-    k_flat_pairs<<<(n_pairs + 255) / 256, 256>>>(t.nodes, n_pairs, eps[0], eps[1], eps[2], pairs, fpairs, flags);
+    k_flat_pairs<<<(n_pairs + 255) / 256, 256>>>(t.nodes, n_pairs, eps[0], eps[1], eps[2], ordered, pairs, fpairs,
+                                                 flags);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpy(got, flags, sizeof got, cudaMemcpyDeviceToHost);
   cudaFreeAsync(flags, 0);

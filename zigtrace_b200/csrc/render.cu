@@ -309,8 +309,8 @@ static zt_status upload_flattened(zt_scene* s, int dev) {
     uint32_t max_leaf = 0;
     bool nan = false;
     if (e == cudaSuccess)
-      rc = flatten_on_device(t, (uint32_t)n, (uint32_t)nn, f.fast_eps, (DPrim*)(b + h->off_prims),
-                             (int32_t*)(b + h->off_ids), (DPair*)(b + h->off_pairs),
+      rc = flatten_on_device(t, (uint32_t)n, (uint32_t)nn, f.fast_eps, s->leaves_ordered,
+                             (DPrim*)(b + h->off_prims), (int32_t*)(b + h->off_ids), (DPair*)(b + h->off_pairs),
                              f.view.fast_ok ? (FPair*)(b + h->off_fpairs) : nullptr, &max_leaf, &nan);
     if (s->nodes[0].count > kFastMaxLeaf) f.view.fast_ok = 0;
     if (nan) f.view.verify_ok = 0;
@@ -425,16 +425,16 @@ __device__ __forceinline__ bool render_pixel(const DevScene& sc, const RenderPar
   const double inv_spp = 1.0 / (double)p.spp;
   Rng rng = rng_for_stream(p.seed, y * p.width + x);
   dv3 sum = V(0, 0, 0);
-  bool unsure = false;
+  int32_t doubt = 0;
   typedef typename Counter<kWalk>::type Count;
   for (Count i = 0; i < (Count)p.spp; ++i) {
     const double s = ((double)x + rng_float(rng)) / w;
     const double t = ((double)y + rng_float(rng)) / h;
     dv3 ro, rd;
     camera_ray(p.cam, s, t, rng, ro, rd);
-    const dv3 c = trace_with<kAux, kNee, kWalk>(sc, ro, rd, rng, p.max_depth, p.use_nee != 0, aux, unsure);
+    const dv3 c = trace_with<kAux, kNee, kWalk>(sc, ro, rd, rng, p.max_depth, p.use_nee != 0, aux, doubt);
     if (kAux) break;
-    if (kWalk != kWalkF64 && unsure) return false;
+    if (kWalk != kWalkF64 && doubt) return false;
     if (visfinite(c)) sum = sum + c;
   }
   if (!kAux) {
@@ -447,7 +447,7 @@ __device__ __forceinline__ bool render_pixel(const DevScene& sc, const RenderPar
   return true;
 }
 
-/* The pixel with the f64 walk, called where the float walk was unsure. */
+/* The pixel with the f64 walk, called where the float walk left it in doubt. */
 __device__ __noinline__ void render_pixel_f64(const DevScene& sc, const RenderParams& p, uint64_t pix,
                                               double* __restrict__ out) {
   render_pixel<false, true, kWalkF64>(sc, p, pix, out, nullptr);
@@ -529,7 +529,8 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
   Rng rng = rng_for_stream(p.seed, valid ? y * p.width + x : 0);
   dv3 sum = V(0, 0, 0);
   uint64_t sample = 0, depth = 0;
-  bool done = !valid, fresh = valid, unsure = false;
+  bool done = !valid, fresh = valid;
+  int32_t doubt = 0;
   /* prev_origin (render.zig:66-70) is read only after a bounce, where it
    * equals ro: ro stands in for it, as in trace_with */
   dv3 ro = V(0, 0, 0), rd = V(0, 0, 0), radiance = V(0, 0, 0), throughput = V(1, 1, 1);
@@ -555,7 +556,7 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
     bool end = depth >= p.max_depth;
     if (!end) {
       Hit hit;
-      if (!scene_intersect<kWalk>(sc, ro, rd, kRayEpsilon, INFINITY, hit, unsure)) {
+      if (!scene_intersect<kWalk>(sc, ro, rd, kRayEpsilon, INFINITY, hit, doubt)) {
         radiance = radiance + vmul(throughput, background_radiance(sc.bg, rd));
         end = true;
       } else {
@@ -567,7 +568,7 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
           radiance = radiance + vscale(vmul(throughput, le), wt);
         }
         if (mat.kind == kLambertian && use_nee)
-          radiance = radiance + vmul(throughput, direct_light<kWalk>(sc, L3(mat.color), hit, rng, unsure));
+          radiance = radiance + vmul(throughput, direct_light<kWalk>(sc, L3(mat.color), hit, rng, doubt));
         dv3 atten, sd;
         if (!material_scatter(mat, rd, hit, rng, atten, sd)) {
           end = true;
@@ -590,10 +591,10 @@ __device__ __forceinline__ void render_pixel_regen(const DevScene& sc, const Ren
       if (visfinite(radiance)) sum = sum + radiance;
       ++sample;
       fresh = true;
-      if (kWalk != kWalkF64 && unsure) sample = p.spp; /* give the pixel up: rendered again below */
+      if (kWalk != kWalkF64 && doubt) sample = p.spp; /* give the pixel up: rendered again below */
     }
   }
-  if (kWalk != kWalkF64 && unsure) {
+  if (kWalk != kWalkF64 && doubt) {
     render_pixel_f64(sc, p, y * p.width + x, out);
   } else if (valid) {
     const dv3 px = vscale(sum, 1.0 / (double)p.spp);
@@ -998,8 +999,9 @@ __global__ void k_trace_paths(DevScene sc, double ox, double oy, double oz, doub
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   Rng rng{rng_state[0], rng_state[1], rng_state[2], rng_state[3]};
   for (uint64_t i = 0; i < n; ++i) {
-    bool unsure = false;
-    const dv3 c = trace_with<false, true, kWalkF64>(sc, V(ox, oy, oz), V(dx, dy, dz), rng, max_depth, use_nee != 0, nullptr, unsure);
+    int32_t doubt = 0;
+    const dv3 c = trace_with<false, true, kWalkF64>(sc, V(ox, oy, oz), V(dx, dy, dz), rng, max_depth, use_nee != 0,
+                                                    nullptr, doubt);
     out[3 * i + 0] = c.x;
     out[3 * i + 1] = c.y;
     out[3 * i + 2] = c.z;

@@ -326,7 +326,7 @@ zt_status build_scene(zt_scene* s, bool device, bool* used_device, double* build
       if (rc == ZT_OK && used_device) *used_device = true;
     }
     if (rc == ZT_DEVICE_BUILD_FALLBACK) rc = build_bvh(s);
-    s->boxes_nested = true;
+    s->boxes_nested = s->leaves_ordered = true;
     if (rc == ZT_OK) rc = build_lights(s);
   } catch (const std::bad_alloc&) {
     return fail(ZT_ERR_OUT_OF_MEMORY, "OutOfMemory during Scene.build");
@@ -352,6 +352,22 @@ static bool boxes_nested(const zt_scene* s) {
     for (uint32_t k = n.first; k < n.first + n.count; ++k) {
       Box b = box_empty();
       if (!shape_bounds(s->shapes[s->indices[k]], b) || !holds(n, b.mn, b.mx)) return false;
+    }
+  }
+  return true;
+}
+
+/* Whether every subtree's primitives are a run of `indices`, the left child's
+ * before the right one's (true of every tree Bvh.build makes). */
+static bool leaves_ordered(const zt_scene* s) {
+  std::vector<std::pair<uint32_t, uint32_t>> run(s->nodes.size()); /* first, end */
+  for (size_t i = s->nodes.size(); i-- > 0;) { /* children follow their parent */
+    const HostNode& n = s->nodes[i];
+    if (n.count > 0) {
+      run[i] = {n.first, n.first + n.count};
+    } else {
+      if (run[n.first].second != run[n.first + 1].first) return false;
+      run[i] = {run[n.first].first, run[n.first + 1].second};
     }
   }
   return true;
@@ -430,6 +446,7 @@ zt_status import_bvh(zt_scene* s, const zt_bvh_node* nodes, size_t n_nodes, cons
     }
     s->indices.assign(indices, indices + n);
     s->boxes_nested = boxes_nested(s);
+    s->leaves_ordered = leaves_ordered(s);
     const zt_status rc = build_lights(s);
     if (rc != ZT_OK) return rc;
   } catch (const std::bad_alloc&) {
@@ -556,6 +573,12 @@ static void make_fast_records(const zt_scene* s, FlatScene* f, bool with_tree) {
         pr.b[c][k][1] = f32_up(ch.bmax[k] + eps[k]);
       }
       pr.word[c] = word(nd.first + c);
+    }
+    pr.split = kNoSplit;
+    if (s->leaves_ordered) {
+      uint32_t at = nd.first + 1;
+      while (s->nodes[at].count == 0) at = s->nodes[at].first;
+      pr.split = s->nodes[at].first;
     }
   }
   for (int k = 0; k < 3; ++k) {

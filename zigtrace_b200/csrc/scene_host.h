@@ -106,6 +106,7 @@ struct zt_scene {
   zt::Array<zt::HostNode> nodes;
   zt::Array<uint32_t> indices;
   bool boxes_nested = false;  /* every node's box holds its children's and its primitives' boxes */
+  bool leaves_ordered = false; /* a left child's primitives come right before its sibling's in `indices` */
   std::vector<zt::HostLight> lights;
   std::vector<double> cdf;
   double total = 0;
@@ -151,10 +152,11 @@ void release_device_tree(zt_scene* s);
 /* The tree a device build left on the current device, if it did. */
 bool device_tree(const zt_scene* s, DeviceTree* out);
 /* Fills the tree's part of the device layout from t on the legacy default
- * stream: the same bytes as flatten_scene's.  fpairs may be NULL.
+ * stream: the same bytes as flatten_scene's.  fpairs may be NULL; ordered:
+ * the scene's leaves_ordered.
  * *max_leaf: the largest leaf; *nan: a primitive holds a NaN. */
-zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_nodes, const double eps[3], DPrim* prims,
-                            int32_t* ids, DPair* pairs, FPair* fpairs, uint32_t* max_leaf, bool* nan);
+zt_status flatten_on_device(const DeviceTree& t, uint32_t n_prims, uint32_t n_nodes, const double eps[3], bool ordered,
+                            DPrim* prims, int32_t* ids, DPair* pairs, FPair* fpairs, uint32_t* max_leaf, bool* nan);
 /* Drops the resident device copy (implemented with the CUDA code). */
 void release_device(zt_scene* s);
 /* Drops the device copy and the pinned staging copy (scene changed). */

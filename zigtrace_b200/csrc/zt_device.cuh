@@ -443,7 +443,7 @@ namespace zt {
 
 /* How a kernel instance walks the tree.  kWalkFloatChecked is the float walk
  * with every hit checked against what the f64 walk would find; where that
- * cannot be shown it sets `unsure`, and the caller renders the pixel again
+ * cannot be shown it sets `doubt`, and the caller renders the pixel again
  * with the f64 walk. */
 enum Walk : int { kWalkF64 = 0, kWalkFloat = 1, kWalkFloatChecked = 2 };
 
@@ -457,15 +457,19 @@ struct Counter<kWalkF64> { typedef uint64_t type; };
 
 /* Closest hit with the hit record. */
 template <int kWalk>
-ZT_D bool scene_intersect(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax, Hit& out, bool& unsure) {
+ZT_D bool scene_intersect(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax, Hit& out, int32_t& doubt) {
   double t;
-  const int32_t k = kWalk != kWalkF64
-                        ? scene_query_fast<kWalk == kWalkFloatChecked>(sc, o, d, tmin, tmax, t, unsure)
-                        : scene_query<false>(sc, o, d, tmin, tmax, t);
+  int32_t k = kWalk != kWalkF64 ? scene_query_fast<kWalk == kWalkFloatChecked>(sc, o, d, tmin, tmax, t, doubt)
+                                : scene_query<false>(sc, o, d, tmin, tmax, t);
   if (k == -1) return false;
   out.t = t;
+  if (kWalk == kWalkFloatChecked && doubt > 0) { /* primitive doubt - 1 is hit at t as well */
+    const int32_t first = tie_first(sc, o, d, tmin, t, k, doubt - 1);
+    if (first >= 0) k = first;
+    doubt = first >= 0 ? 0 : -1;
+  }
   hit_from(sc, k, o, d, t, out);
-  if (kWalk == kWalkFloatChecked && k >= 0 && !walk_reaches(sc, sc.prims[k], o, out.point)) unsure = true;
+  if (kWalk == kWalkFloatChecked && k >= 0 && !walk_reaches(sc, sc.prims[k], o, out.point)) doubt = -1;
   return true;
 }
 
@@ -714,7 +718,7 @@ ZT_D double power_weight(double a, double b) { /* render.zig:38-41 */
 
 /* directLight, render.zig:46-56 (shadow ray as an any-hit query). */
 template <int kWalk>
-ZT_D dv3 direct_light(const DevScene& sc, dv3 albedo, const Hit& hit, Rng& rng, bool& unsure) {
+ZT_D dv3 direct_light(const DevScene& sc, dv3 albedo, const Hit& hit, Rng& rng, int32_t& doubt) {
   dv3 ldir, lrad;
   double ldist, lpdf;
   if (!lights_sample<kWalk != kWalkF64>(sc, hit.point, rng, ldir, ldist, lrad, lpdf)) return V(0, 0, 0);
@@ -722,7 +726,7 @@ ZT_D dv3 direct_light(const DevScene& sc, dv3 albedo, const Hit& hit, Rng& rng, 
   if (cos_s <= 0 || !(lpdf > 0)) return V(0, 0, 0);
   const double shadow_tmax = ldist * (1 - 1e-6);
   if (kWalk != kWalkF64
-          ? scene_occluded_fast<kWalk == kWalkFloatChecked>(sc, hit.point, ldir, kRayEpsilon, shadow_tmax, unsure)
+          ? scene_occluded_fast<kWalk == kWalkFloatChecked>(sc, hit.point, ldir, kRayEpsilon, shadow_tmax, doubt)
           : scene_occluded(sc, hit.point, ldir, kRayEpsilon, shadow_tmax))
     return V(0, 0, 0);
   const double bsdf_pdf = cos_s / kPi;
@@ -737,7 +741,7 @@ struct TraceAux { int32_t first_prim; uint32_t path_len; };
 
 template <bool kAux, bool kNee, int kWalk>
 ZT_D dv3 trace_with(const DevScene& sc, dv3 ro, dv3 rd, Rng& rng, uint64_t max_depth, bool use_nee_arg,
-                    TraceAux* aux, bool& unsure) {
+                    TraceAux* aux, int32_t& doubt) {
   const bool use_nee = kNee && use_nee_arg;
   /* The reference's prev_origin (render.zig:66-70) is read only when
    * prev_pdf > 0, i.e. after a bounce, where it always equals the current
@@ -751,7 +755,7 @@ ZT_D dv3 trace_with(const DevScene& sc, dv3 ro, dv3 rd, Rng& rng, uint64_t max_d
   for (Count depth = 0; depth < (Count)max_depth; ++depth) {
     Hit hit;
     if (kAux) n_ext++;
-    if (!scene_intersect<kWalk>(sc, ro, rd, kRayEpsilon, INFINITY, hit, unsure)) {
+    if (!scene_intersect<kWalk>(sc, ro, rd, kRayEpsilon, INFINITY, hit, doubt)) {
       if (kAux) aux->path_len = n_ext;
       return radiance + vmul(throughput, background_radiance(sc.bg, rd));
     }
@@ -764,7 +768,7 @@ ZT_D dv3 trace_with(const DevScene& sc, dv3 ro, dv3 rd, Rng& rng, uint64_t max_d
       radiance = radiance + vscale(vmul(throughput, le), w);
     }
     if (mat.kind == kLambertian && use_nee)
-      radiance = radiance + vmul(throughput, direct_light<kWalk>(sc, L3(mat.color), hit, rng, unsure));
+      radiance = radiance + vmul(throughput, direct_light<kWalk>(sc, L3(mat.color), hit, rng, doubt));
     dv3 atten, sd;
     if (!material_scatter(mat, rd, hit, rng, atten, sd)) break;
     throughput = vmul(throughput, atten);

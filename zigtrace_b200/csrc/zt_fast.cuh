@@ -60,11 +60,13 @@
  * its results are the f64 walk's bit for bit:
  *  - a tie: another primitive is hit at exactly the closest distance.  In
  *    one leaf both walks test the primitives in the same order and the first
- *    keeps the hit; only a tie between leaves is in doubt.  (Coincident
- *    primitives have one centroid, which no split separates.  With every tie
- *    in doubt, the 250k-triangle terrain 961x541x16 with each triangle twice
- *    took 21.0 ms, with each fiftieth twice 22.6; now 13.8 and 10.6, the f64
- *    walk alone 17.3 and 14.0.)
+ *    keeps the hit (coincident primitives have one centroid, which no split
+ *    separates); between two leaves the f64 walk's order of visiting them is
+ *    worked out (tie_first); a third primitive at the distance leaves a doubt.
+ *    With every tie in doubt, the 250k-triangle terrain 961x541x16 with each
+ *    fiftieth triangle twice took 22.6 ms, now 10.6, with the f64 walk alone
+ *    14.0; a closed box of 2,572 triangles with its light in the plane of its
+ *    ceiling, 800x800x32, 122 ms, 40.2 and 39.8;
  *  - a hit whose leaf the f64 walk might miss: walk_reaches shows that the
  *    hit point lies inside the primitive's box by more than the f64 test's
  *    rounding.  Every ancestor's box holds that box (boxes_nested), so the
@@ -72,7 +74,7 @@
  *    exceeds the hit's, so no pop is pruned: the f64 walk tests the
  *    primitive, and it is the least hit of a superset of what that walk
  *    tests.  No hit in the superset means none in the f64 walk.
- * Where either is in doubt `unsure` is set and the caller renders the pixel
+ * Where either is in doubt `doubt` is set and the caller renders the pixel
  * again with the f64 walk (none of the images measured below: the flag costs
  * a register, where a call of the f64 walk from inside this one measured 7% on
  * the 1M-triangle terrain and 12% on the sphere fields).  Rays the float
@@ -133,7 +135,7 @@ ZT_D float fmin3f(float a, float b, float c) {
 
 /* Largest |origin| (component sum) the float test takes (derived above).
  * Rays from farther away (a hit far out on an unbounded plane), with a NaN, or
- * with a direction far from unit length make the pixel unsure. */
+ * with a direction far from unit length leave the pixel in doubt. */
 constexpr float kFastMaxOrigin = 1e10f;
 
 ZT_D bool fray_make(dv3 o, dv3 d, FRay& r) {
@@ -181,6 +183,35 @@ ZT_D bool walk_reaches(const DevScene& sc, const DPrim& p, dv3 o, dv3 point) {
   return reach_inside(p.kind == kTriangle, p.a, h.x, h.y, h.z, m);
 }
 
+/* Which of two primitives of different leaves, a and b, hit at the same
+ * distance t, the f64 walk tests first and so keeps; -1 where that cannot be
+ * shown.  Both hits must be certain to be reached (walk_reaches); the walk then
+ * enters both children of the lowest node above the two leaves, the nearer one
+ * first, and finishes with it before the other.  The node is found from the
+ * root by the records' splits, and its children's entry distances are the f64
+ * walk's own (slab).  A call, and its result by value: inlined, random spheres
+ * took 4.00 ms against 3.86. */
+__device__ __noinline__ int32_t tie_first(const DevScene& sc, dv3 o, dv3 d, double tmin, double t, int32_t a,
+                                          int32_t b) {
+  const dv3 point = o + vscale(d, t);
+  if (!walk_reaches(sc, sc.prims[a], o, point) || !walk_reaches(sc, sc.prims[b], o, point)) return -1;
+  uint32_t w = sc.froot_word;
+  bool a_right;
+  for (;;) {
+    if (w >> kFastCountShift) return -1; /* no order to go by (kNoSplit) */
+    const FPair& r = sc.fpairs[w];
+    a_right = (uint32_t)a >= r.split;
+    if (a_right != ((uint32_t)b >= r.split)) break;
+    w = r.word[a_right];
+  }
+  const DPair& p = sc.pairs[w];
+  const dv3 inv = V(1.0 / d.x, 1.0 / d.y, 1.0 / d.z);
+  double tl, tr;
+  slab(p.lo[0], p.hi[0], o, inv, tmin, t, tl);
+  slab(p.lo[1], p.hi[1], o, inv, tmin, t, tr);
+  return (tl <= tr) != a_right ? a : b;
+}
+
 /* One 64-byte record: both children's axis pairs and payload words. */
 struct FRec {
   ulonglong2 q0, q1, q2;
@@ -211,17 +242,19 @@ ZT_D bool fslab_root(const DevScene& sc, const FRay& fr, float tmin, float tmax,
  * records: nearest first by float entry distance (ties to the left child,
  * bvh.zig:111-116), pruning entries whose distance exceeds the closest hit,
  * f64 primitive tests; then the unbounded planes.  Return value and t_out as
- * scene_query_rt's (closest hit only).  kVerify notes ties in `unsure`; the
- * caller checks the hit itself with walk_reaches, beside its hit record. */
+ * scene_query_rt's (closest hit only).  kVerify notes what is in doubt (0:
+ * nothing, k + 1: primitive k ties with the hit, -1: the f64 walk has to
+ * decide); the caller checks the hit itself with walk_reaches, beside its hit
+ * record. */
 template <bool kVerify>
 ZT_D int32_t scene_query_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax, double& t_out,
-                              bool& unsure) {
+                              int32_t& doubt) {
   double closest = tmax;
   int32_t best_k = -1;
   if (sc.has_root) {
     FRay fr;
     if (!fray_make(o, d, fr)) {
-      unsure = true;
+      doubt = -1;
       return -1;
     }
     const float tmin32 = __double2float_rd(tmin);
@@ -244,21 +277,28 @@ ZT_D int32_t scene_query_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, dou
         if (et > cl32) continue; /* bvh.zig:97, against closest rounded up */
         const uint32_t cnt = w >> kFastCountShift, first = w & kFastFirstMask;
         if (cnt > 0) {
-          /* in a leaf a hit of its own is kept as -2 - k (with a flag beside it terrain 11.2 ms against 11.05) */
-          for (uint32_t k = first; k < first + cnt; ++k) {
+          /* One word counts the leaf's primitives off and holds the next one's index; in a leaf a hit of its own is
+           * kept as -2 - k.  (With an end index the 256 sphere fields took 52.6 ms, so 51.9, with
+           * ZT_PRECISION_FAST 51.3 and 50.5.) */
+          uint32_t left = w;
+          do {
+            const uint32_t k = left & kFastFirstMask;
             double th;
             if (bounded_t<kVerify>(sc.prims[k], o, d, tmin, closest, th)) {
               if (kVerify && !(th < closest)) {
                 /* a tie (or a NaN): in one leaf the first primitive keeps the hit, as in the f64 walk; between
-                 * leaves that walk's visiting order decides */
-                if (best_k >= -1 || !(th == closest)) unsure = true;
+                 * leaves that walk's visiting order decides (tie_first) */
+                if (best_k >= -1 || !(th == closest))
+                  doubt = best_k >= 0 && th == closest && doubt == 0 ? (int32_t)k + 1 : -1;
               } else {
                 closest = th;
                 best_k = kVerify ? -2 - (int32_t)k : (int32_t)k;
                 cl32 = __double2float_ru(th);
+                if (kVerify) doubt = min(doubt, 0); /* ties behind the hit are of no account */
               }
             }
-          }
+            left += 1u - (1u << kFastCountShift);
+          } while (left >> kFastCountShift);
           if (kVerify && best_k < -1) best_k = -2 - best_k;
           continue;
         }
@@ -286,6 +326,7 @@ ZT_D int32_t scene_query_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, dou
     if (plane_prim_t(sc.planes[i], o, d, tmin, closest, th)) {
       closest = th;
       best_k = -2 - (int32_t)i;
+      if (kVerify) doubt = min(doubt, 0);
     }
   }
   t_out = closest;
@@ -298,11 +339,11 @@ ZT_D int32_t scene_query_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, dou
  * finds it; kVerify checks that the f64 walk reaches the one found.  Farther
  * child first, as scene_occluded. */
 template <bool kVerify>
-ZT_D bool scene_occluded_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax, bool& unsure) {
+ZT_D bool scene_occluded_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, double tmax, int32_t& doubt) {
   if (sc.has_root) {
     FRay fr;
     if (!fray_make(o, d, fr)) {
-      unsure = true;
+      doubt = -1;
       return true;
     }
     const float tmin32 = __double2float_rd(tmin), tmax32 = __double2float_ru(tmax);
@@ -323,7 +364,7 @@ ZT_D bool scene_occluded_fast(const DevScene& sc, dv3 o, dv3 d, double tmin, dou
           for (uint32_t k = first; k < first + cnt; ++k) {
             double th;
             if (prim_t(sc.prims[k], o, d, tmin, tmax, th)) {
-              if (kVerify && !walk_reaches(sc, sc.prims[k], o, o + vscale(d, th))) unsure = true;
+              if (kVerify && !walk_reaches(sc, sc.prims[k], o, o + vscale(d, th))) doubt = -1;
               return true;
             }
           }

@@ -64,10 +64,12 @@ struct ZT_ALIGN(128) DPair {
 struct ZT_ALIGN(64) FPair {
   float b[2][3][2]; /* [child][axis][lower, upper] */
   uint32_t word[2];
-  uint32_t pad[2];
+  uint32_t split; /* first primitive of the right child; kNoSplit where the leaves are not in the tree's order */
+  uint32_t pad;
 };
 constexpr uint32_t kFastCountShift = 28;
 constexpr uint32_t kFastFirstMask = (1u << kFastCountShift) - 1;
+constexpr uint32_t kNoSplit = 0xFFFFFFFFu;
 constexpr uint32_t kFastMaxLeaf = (1u << (32 - kFastCountShift)) - 1;
 /* Largest |coordinate| (of the scene's bounds and of ray origins) the float
  * slab test handles: products with the clamped reciprocal stay finite. */
