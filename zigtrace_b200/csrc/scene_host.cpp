@@ -35,6 +35,7 @@ zt_status fail(zt_status code, const std::string& msg) {
  * started, the caller does the work.  f must not throw. */
 template <typename F>
 static void parallel_ranges(size_t n, size_t grain, const F& f) {
+  if (n < 2 * grain) return f((size_t)0, n); /* not even asking for the number of cores, which takes some microseconds */
   const size_t cores = std::max(1u, std::thread::hardware_concurrency());
   const size_t parts = std::max<size_t>(1, std::min({n / grain, cores, (size_t)8}));
   std::thread team[8];
