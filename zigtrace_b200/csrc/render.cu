@@ -1040,6 +1040,10 @@ static unsigned persistent_grid(K kernel, int block, uint64_t work_items, size_t
 enum MegaVariant { kMegaNested = 0, kMegaRegen = 1 };
 constexpr double kRegenMeanPath = 3.0;
 
+/* Bounded primitives from which a single render takes the float walk
+ * (choose_walk). */
+constexpr uint32_t kFastMinPrimitives = 64;
+
 /* Parts per tile (log2) of a render with few pixels.  A warp renders its
  * tile's pixels as long as the longest of their paths takes at every bounce,
  * so a part of the tile is done sooner than the whole; where the tiles do not
@@ -1069,22 +1073,30 @@ static uint32_t choose_split(const RenderParams& p, uint64_t room) {
 /* Of the kernels with path regeneration (512 threads per SM). */
 static uint64_t regen_room() { return (uint64_t)sm_count() * (512 / 32) * 3 / 8; }
 
+/* Of the nested instances.  Below kFastMinPrimitives the walks of a warp
+ * differ little and its f64 work is what the SM is busy with, so more warps
+ * slow it down as they do the regeneration instance (Cornell box, nested
+ * kernel 256x256x16: whole tiles 2.94 ms, in halves 3.36). */
+static uint64_t nested_room(uint32_t n_prims, int threads_per_sm) {
+  const uint64_t resident = (uint64_t)sm_count() * threads_per_sm / 32;
+  return n_prims < kFastMinPrimitives ? resident * 3 / 8 : n_prims >= 4096 ? 2 * resident : resident;
+}
+
 template <int BS, int kWalk>
 static void launch_mega_bsf(const DevScene& v, const RenderParams& params, double* d_out, unsigned int* counter,
                             MegaVariant variant, cudaStream_t stream) {
   RenderParams p = params;
-  const uint64_t sms = (uint64_t)sm_count() * (v.n_prims >= 4096 ? 2 : 1);
   if (variant == kMegaRegen) {
     p.split = choose_split(p, regen_room());
     k_render_regen<BS, kWalk><<<persistent_grid(k_render_regen<BS, kWalk>, BS, work_units(p) * 32), BS, 0, stream>>>(
         v, p, d_out, counter);
   } else if (p.use_nee) {
-    p.split = choose_split(p, sms * mega_threads_per_sm(true, kWalk) / 32);
+    p.split = choose_split(p, nested_room(v.n_prims, mega_threads_per_sm(true, kWalk)));
     k_render_mega<BS, true, kWalk>
         <<<persistent_grid(k_render_mega<BS, true, kWalk>, BS, work_units(p) * 32), BS, 0, stream>>>(v, p, d_out,
                                                                                                   counter);
   } else {
-    p.split = choose_split(p, sms * mega_threads_per_sm(false, kWalk) / 32);
+    p.split = choose_split(p, nested_room(v.n_prims, mega_threads_per_sm(false, kWalk)));
     k_render_mega<BS, false, kWalk>
         <<<persistent_grid(k_render_mega<BS, false, kWalk>, BS, work_units(p) * 32), BS, 0, stream>>>(v, p, d_out,
                                                                                                    counter);
@@ -1109,7 +1121,6 @@ static bool valid_block_size(uint32_t bs) { return bs == 0 || bs == 64 || bs == 
  * than its box tests save (Cornell box, 14 primitives: 477 against 565
  * Msamples/s); a batch, whose renders share one kernel instance, weighs its
  * scenes (zt_batch_create). */
-constexpr uint32_t kFastMinPrimitives = 64;
 static Walk choose_walk(const zt_scene* s, const RenderParams& p, uint32_t precision, bool small_scenes_f64 = true) {
   if (!s->device || !s->device->view.fast_ok) return kWalkF64;
   if (p.spp > 0xFFFFFFFFull || p.max_depth > 0xFFFFFFFFull) return kWalkF64; /* 32-bit counters */
