@@ -1649,14 +1649,16 @@ zt_status zt_rng_streams(uint64_t seed, uint64_t stream0, uint64_t n_streams, ui
 /* --------------------------------------------------- Differentiable form ---- */
 namespace zt {
 
-/* Forward of the detached estimator (zt_diff.cuh): the megakernel's tile loop
- * with per-lane path regeneration (render_pixel_regen: a lane whose path ends
- * starts its pixel's next sample at once); theta == the scene's colours gives
- * zt_render's image.  sample_L (may be NULL) keeps every sample's radiance
- * for zt_backward.  Built for four blocks of 128 per SM (128 registers):
- * 512x512x64 of the Cornell-style box 25.3 ms, at five blocks 26.1, nested
- * (every lane waiting for the warp's longest path) 28.4. */
-template <int BS>
+/* Forward of the detached estimator (zt_diff.cuh): the megakernel's tile loop,
+ * nested or with per-lane path regeneration (render_pixel_regen: a lane whose
+ * path ends starts its pixel's next sample at once), as the scene's paths ask
+ * for (kRegenMeanPath); theta == the scene's colours gives zt_render's image.
+ * sample_L (may be NULL) keeps every sample's radiance for zt_backward.  Built
+ * for four blocks of 128 per SM (128 registers): 512x512x64 of the Cornell-style
+ * box 25.3 ms, at five blocks 26.1, nested (every lane waiting for the warp's
+ * longest path) 28.4; 320 random spheres 160x90x16 0.88 nested against 1.05,
+ * 66k-triangle terrain 3.1 against 7.0. */
+template <int BS, bool kRegen>
 __global__ void __launch_bounds__(BS, 512 / BS) k_forward_diff(const __grid_constant__ DevScene sc,
                                                              const __grid_constant__ RenderParams p,
                                                              const double* __restrict__ theta,
@@ -1690,9 +1692,13 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_forward_diff(const __grid_cons
       }
       if (__all_sync(0xffffffffu, done)) break;
       if (done) continue;
-      const bool end = diff_bounce(sc, theta, s, depth, rng, p.use_nee != 0, false, V(0, 0, 0), V(0, 0, 0), nullptr);
-      depth += 1;
-      if (end || depth >= p.max_depth) {
+      bool end;
+      do { /* one bounce, or the whole path */
+        end = diff_bounce(sc, theta, s, depth, rng, p.use_nee != 0, false, V(0, 0, 0), V(0, 0, 0), nullptr);
+        depth += 1;
+        end = end || depth >= p.max_depth;
+      } while (!kRegen && !end);
+      if (end) {
         if (sample_L) {
           double* q = sample_L + 3 * (sample * p.width * p.height + pix);
           q[0] = s.radiance.x;
@@ -1851,7 +1857,8 @@ zt_status zt_forward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin, 
   RenderParams p = make_params(s, o);
   p.row0 = row_begin;
   p.rows = row_end - row_begin;
-  p.split = choose_split(p, regen_room());
+  const bool regen = s->pilot_valid && s->mean_path >= kRegenMeanPath;
+  p.split = choose_split(p, regen ? regen_room() : nested_room(s->device->view.n_prims, 512));
   const size_t bytes = (size_t)(p.rows * o->width * 3) * sizeof(double);
   zt_diff_cache& cache = s->device->diff;
   cache.valid = false;
@@ -1883,8 +1890,12 @@ zt_status zt_forward_rows(zt_scene* s, const zt_options* o, uint64_t row_begin, 
   }
   cudaError_t e = cudaMemsetAsync(s->device->counter, 0, sizeof(unsigned int), 0);
   if (e == cudaSuccess) {
-    k_forward_diff<128><<<persistent_grid(k_forward_diff<128>, 128, work_units(p) * 32), 128>>>(
-        launch_view(s), p, d_theta, d_out, cache.L, s->device->counter);
+    if (regen)
+      k_forward_diff<128, true><<<persistent_grid(k_forward_diff<128, true>, 128, work_units(p) * 32), 128>>>(
+          launch_view(s), p, d_theta, d_out, cache.L, s->device->counter);
+    else
+      k_forward_diff<128, false><<<persistent_grid(k_forward_diff<128, false>, 128, work_units(p) * 32), 128>>>(
+          launch_view(s), p, d_theta, d_out, cache.L, s->device->counter);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpy(out, d_out, bytes, cudaMemcpyDeviceToHost);
