@@ -1113,10 +1113,36 @@ static void launch_mega_bs(const DevScene& v, const RenderParams& p, double* d_o
 
 static bool valid_block_size(uint32_t bs) { return bs == 0 || bs == 64 || bs == 128 || bs == 256; }
 
+/* Whether the float boxes are so much larger than the scene's leaves that the
+ * f64 walk is the faster one.  Records are widened by 2^-20 of the scene's
+ * reach and rays by 2^-20 of their origin's (zt_fast.cuh): on a ground a
+ * million times the size of what stands on it that is more than the objects
+ * are apart, and every ray visits most of them.  The line lies where a typical
+ * leaf's area has grown by kCoarseArea, and for camera rays, of which a path
+ * has one, from a distant camera, by kCoarseAreaCamera.  Measured, float walk
+ * against f64 walk: 66k-triangle terrain on a square of half side 1e4 (area x
+ * 1.06) 8.7 against 10.8 ms, 1e5 (1.7) 10.6 and 10.7, 2e5 (2.6) 13.5 and 10.7,
+ * 1e6 (17) 50.6 and 10.8; random spheres on such squares 1e5 (1.7) 4.2 and
+ * 5.7, 2e5 (2.6) 4.4 and 5.7, 1e6 (15) 6.5 and 5.7, 9e6 (670) 66 and 5.7;
+ * random spheres seen from 1e5 (2.2) 2.3 and 2.8, 1e6 (33) 4.7 and 4.4, 9e6
+ * 8.3 and 4.1.  ZT_PRECISION_FAST walks the float boxes all the same. */
+constexpr double kCoarseArea = 1.8, kCoarseAreaCamera = 4;
+static bool float_boxes_coarse(const zt_scene* s, const double camera[3], double around) {
+  const DevScene& v = s->device->view;
+  const double* e = s->leaf_extent;
+  double f[3], g[3]; /* widened by the record's margin, and by the camera ray's as well */
+  for (int k = 0; k < 3; ++k) {
+    f[k] = e[k] + ldexp(fmax(fabs(v.root_lo[k]), fabs(v.root_hi[k])), -19);
+    g[k] = f[k] + ldexp(fabs(camera[k]) + around, -19);
+  }
+  auto area = [](const double* x) { return x[0] * x[1] + x[1] * x[2] + x[2] * x[0]; };
+  return area(f) > kCoarseArea * area(e) || area(g) > kCoarseAreaCamera * area(e);
+}
+
 /* The walk a render takes.  The float walk needs the scene's float records
  * and a camera origin within their coordinate range; ZT_PRECISION_EXACT also
- * needs boxes that its hits can be checked against (verify_ok) and walks
- * checked.  A single render needs at least kFastMinPrimitives bounded
+ * needs boxes that its hits can be checked against (verify_ok) and that are
+ * not coarse, and walks checked.  A single render needs at least kFastMinPrimitives bounded
  * primitives: on a tree this small the float walk's per-ray set-up costs more
  * than its box tests save (Cornell box, 14 primitives: 477 against 565
  * Msamples/s); a batch, whose renders share one kernel instance, weighs its
@@ -1132,7 +1158,8 @@ static Walk choose_walk(const zt_scene* s, const RenderParams& p, uint32_t preci
   const bool near = fabs(o[0]) + reach <= kFastMaxCoord && fabs(o[1]) + reach <= kFastMaxCoord &&
                     fabs(o[2]) + reach <= kFastMaxCoord;
   if (!near) return kWalkF64;
-  return precision == ZT_PRECISION_FAST ? kWalkFloat : kWalkFloatChecked;
+  if (precision == ZT_PRECISION_FAST) return kWalkFloat;
+  return float_boxes_coarse(s, o, reach) ? kWalkF64 : kWalkFloatChecked;
 }
 
 static zt_status launch_mega(zt_scene* s, const RenderParams& p, uint32_t block_size, double* d_out,

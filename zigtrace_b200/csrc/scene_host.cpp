@@ -311,6 +311,21 @@ static zt_status check_materials(const zt_scene* s) {
   return ZT_OK;
 }
 
+/* How large the leaves' boxes are: geometric means over some 256 of them, so
+ * that a ground many times the size of everything else counts for little. */
+static void measure_leaves(zt_scene* s) {
+  const size_t nn = s->nodes.size(), step = (nn / 512) | 1;
+  double sum[3] = {0, 0, 0};
+  size_t n = 0;
+  for (size_t i = 0; i < nn; i += step) {
+    const HostNode& nd = s->nodes[i];
+    if (nd.count == 0) continue;
+    for (int k = 0; k < 3; ++k) sum[k] += std::log2((float)std::max(nd.bmax[k] - nd.bmin[k], 1e-30));
+    ++n;
+  }
+  for (int k = 0; k < 3; ++k) s->leaf_extent[k] = n > 0 ? std::exp2(sum[k] / (double)n) : INFINITY;
+}
+
 zt_status build_scene(zt_scene* s, bool device, bool* used_device, double* build_ms) { /* Scene.build, scene.zig:92-96 */
   const zt_status materials = check_materials(s);
   if (materials != ZT_OK) return materials;
@@ -328,6 +343,7 @@ zt_status build_scene(zt_scene* s, bool device, bool* used_device, double* build
     }
     if (rc == ZT_DEVICE_BUILD_FALLBACK) rc = build_bvh(s);
     s->boxes_nested = s->leaves_ordered = true;
+    measure_leaves(s);
     if (rc == ZT_OK) rc = build_lights(s);
   } catch (const std::bad_alloc&) {
     return fail(ZT_ERR_OUT_OF_MEMORY, "OutOfMemory during Scene.build");
@@ -448,6 +464,7 @@ zt_status import_bvh(zt_scene* s, const zt_bvh_node* nodes, size_t n_nodes, cons
     s->indices.assign(indices, indices + n);
     s->boxes_nested = boxes_nested(s);
     s->leaves_ordered = leaves_ordered(s);
+    measure_leaves(s);
     const zt_status rc = build_lights(s);
     if (rc != ZT_OK) return rc;
   } catch (const std::bad_alloc&) {

@@ -6,6 +6,7 @@
 #ifndef ZT_SCENE_HOST_H
 #define ZT_SCENE_HOST_H
 
+#include <math.h>
 #include <stdlib.h>
 #include <sys/mman.h>
 
@@ -106,6 +107,7 @@ struct zt_scene {
   zt::Array<zt::HostNode> nodes;
   zt::Array<uint32_t> indices;
   bool boxes_nested = false;  /* every node's box holds its children's and its primitives' boxes */
+  double leaf_extent[3] = {INFINITY, INFINITY, INFINITY}; /* of the leaves' boxes, about: geometric means */
   bool leaves_ordered = false; /* a left child's primitives come right before its sibling's in `indices` */
   std::vector<zt::HostLight> lights;
   std::vector<double> cdf;
