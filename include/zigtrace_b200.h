@@ -93,7 +93,9 @@ enum { ZT_MODE_AUTO = 0, ZT_MODE_MEGAKERNEL = 1, ZT_MODE_WAVEFRONT = 2, ZT_MODE_
  * every value is the reference's f64 value, computed in the reference's
  * order (BVH boxes of scenes with 64 or more bounded primitives are tested in
  * single precision first, and every hit so found is checked to be the one the
- * f64 walk finds; pixels where that is in doubt take the f64 walk), so images
+ * f64 walk finds; pixels where that is in doubt take the f64 walk; a triangle
+ * met within some 2e-9 of its plane is the one thing the check rests on but
+ * cannot see), so images
  * are bit-identical to the reference algorithm's as restated by
  * the project's CPU oracle (which shares this library's sin/cos, so parity
  * with Zig's own transcendentals is not covered).

@@ -343,10 +343,11 @@ static zt_status upload_flattened(zt_scene* s, int dev) {
 
 static zt_status pilot_paths(zt_scene* s);
 
-/* Makes the scene resident on the current device.  With sync = false the
- * host-to-device copy is left in flight on the legacy default stream (work
- * later enqueued there, or after a synchronisation, sees it): a caller
- * uploading many scenes synchronises once. */
+/* Makes the scene resident on the current device.  With sync = false the copy
+ * of a scene that has its pinned image is left in flight on the legacy default
+ * stream (work later enqueued there, or after a synchronisation, sees it), so
+ * that a caller uploading many such scenes synchronises once.  A scene's first
+ * uploads, flattened on the device, wait for its flags in any case. */
 static zt_status upload(zt_scene* s, bool sync = true) {
   if (!s->built) return fail(ZT_ERR_NOT_BUILT, "scene is not built: call zt_scene_build first");
   int dev = 0;
@@ -455,7 +456,7 @@ __device__ __noinline__ void render_pixel_f64(const DevScene& sc, const RenderPa
 
 /* The pixel of this lane in work unit `unit`: every 8x4 tile is 2^p.split
  * units, each a rectangle of the tile for the first lanes of the warp (8x4,
- * 4x4, 4x2, 2x2, 2x1 or one pixel).  False: no pixel for this lane. */
+ * 4x4, 4x2, 2x2 or 2x1).  False: no pixel for this lane. */
 __device__ __forceinline__ bool unit_pixel(const RenderParams& p, uint64_t tiles_x, unsigned unit, uint64_t& x,
                                            uint64_t& y) {
   const unsigned lane = threadIdx.x & 31;
@@ -2104,7 +2105,7 @@ zt_status zt_batch_create(zt_scene* const* scenes, const zt_options* opts, uint6
     zt_status rc = check_render_args(scenes[i], &opts[i]);
     if (rc != ZT_OK) return rc;
     if (!d_outs[i]) return fail(ZT_ERR_INVALID_ARGUMENT, "zt_batch_create: NULL output");
-    rc = upload(scenes[i], false); /* copies in flight; one synchronisation below */
+    rc = upload(scenes[i], false); /* copies may be in flight until the synchronisation below */
     if (rc != ZT_OK) return rc;
     idx[i] = i;
     /* expected work: samples x log2 of the primitive count */

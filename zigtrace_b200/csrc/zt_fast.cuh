@@ -22,8 +22,8 @@
  *    reciprocal's 2^-23);
  *  - the |c| part is covered by the records: every bound is moved outward by
  *    eps = 2^-20 M (M the largest |bound| on that axis; 4x the 2 2^-23 M
- *    needed; kFastMinMargin at least), which moves a near plane's distance down and a far plane's up
- *    by eps / |d|;
+ *    needed; kFastMinMargin at least), which moves a near plane's distance
+ *    down and a far plane's up by eps / |d|;
  *  - the |o| part is covered per ray: w = 2^-20 |n| (2.3x the 3.5 2^-23 |o I|
  *    needed) is subtracted from near planes and added to far planes;
  *  - so each near distance is at most the exact one and each far distance at
@@ -46,18 +46,28 @@
  *    ray parallel to an axis was missed from about 3e18 on, and from less in
  *    flat scenes.)
  * Entry distances are lower bounds of the exact ones, so `entry.t > closest`
- * pruning against closest rounded up never drops a node the reference
- * visits, and leaves are tested with the reference's f64 primitive tests.
- * The closest hit found is therefore the least primitive distance over a
- * superset of the leaves the reference tests; it differs from the
- * reference's only where two primitives tie, or where the reference's own
- * f64 box test misses a primitive hit by rounding (a grazing ray).
+ * against closest rounded up drops a node only when the ray enters its box
+ * behind a hit already found, and leaves are tested with the reference's f64
+ * primitive tests.  The closest hit found is therefore the least primitive
+ * distance over a superset of the leaves the reference tests; it differs from
+ * the reference's only
+ *  - where two primitives tie;
+ *  - where the reference's own f64 box test misses a primitive hit by rounding
+ *    (a grazing ray);
+ *  - where a primitive in a dropped node is hit in front of its own box, and the
+ *    reference, which may come to that node before the other hit, tests it.
+ *    The boxes' margins (2^-20 of the coordinates) exceed what a sphere test
+ *    errs by; a triangle's distance errs by 18u (|s| + |e|) |e1||e2| / |det|
+ *    (light_passed in zt_device.cuh), more than the margins only where the ray
+ *    meets the triangle at a cosine below some 2e-9 |e1||e2| / |e1 x e2|.
  * ZT_PRECISION_FAST takes the result as it is: its images are held to a
  * statistical bar (per-channel relative RMSE and mean luminance against the
  * oracle), not to bit equality.
  *
- * The checked walk (kVerify, ZT_PRECISION_EXACT) detects those two cases, so
- * its results are the f64 walk's bit for bit:
+ * The checked walk (kVerify, ZT_PRECISION_EXACT) detects the first two, so its
+ * results are the f64 walk's bit for bit but for the third, which is not
+ * detected and has not been met (a ray within 2e-9 of a triangle's plane, and
+ * another hit within the error of it):
  *  - a tie: another primitive is hit at exactly the closest distance.  In
  *    one leaf both walks test the primitives in the same order and the first
  *    keeps the hit (coincident primitives have one centroid, which no split
@@ -73,7 +83,8 @@
  *    f64 test passes at every node on the way down, and no entry distance
  *    exceeds the hit's, so no pop is pruned: the f64 walk tests the
  *    primitive, and it is the least hit of a superset of what that walk
- *    tests.  No hit in the superset means none in the f64 walk.
+ *    tests (the third case apart).  No hit in the superset means none in the
+ *    f64 walk: nothing is dropped before a first hit.
  * Where either is in doubt `doubt` is set and the caller renders the pixel
  * again with the f64 walk (none of the images measured below: the flag costs
  * a register, where a call of the f64 walk from inside this one measured 7% on
