@@ -37,26 +37,28 @@ NOMINAL_SM_MHZ = 1965.0
 # workload, --clock-control none) and scaled by samples per launch: traffic
 # grows with the samples traced.  Keyed by (workload, precision); workloads
 # without a capture report null.
-NCU_DRAM_BYTES_PER_SAMPLE = {("triangle_heavy", "exact"): (0.944641e9 + 1.011825e9) / (1920 * 1080 * 8),
-                             ("triangle_heavy", "fast"): (0.993070e9 + 1.097135e9) / (1920 * 1080 * 8)}
+NCU_DRAM_BYTES_PER_SAMPLE = {("triangle_heavy", "exact"): (0.922717e9 + 0.989119e9) / (1920 * 1080 * 8),
+                             ("triangle_heavy", "fast"): (0.932459e9 + 1.016554e9) / (1920 * 1080 * 8)}
 # What bounds the kernel instead of a pipe peak, from the same capture:
 # issue slots used, lanes active per warp instruction, FP64 pipe activity.
-NCU_EXECUTION = {("triangle_heavy", "exact"): {"issue_active_pct": 59.7, "lanes_per_warp_instruction": 7.58,
-                                               "fp64_pipe_active_pct": 26.9, "fma_pipe_active_pct": 10.1,
-                                               "l1_hit_pct": 79.3, "l2_hit_pct": 84.7,
-                                               "top_stall": "long_scoreboard 5.3 cycles per issue"},
-                 ("triangle_heavy", "fast"): {"issue_active_pct": 60.2, "lanes_per_warp_instruction": 7.59,
-                                              "fp64_pipe_active_pct": 27.4, "fma_pipe_active_pct": 10.1,
-                                              "l1_hit_pct": 78.6, "l2_hit_pct": 84.3,
-                                              "top_stall": "long_scoreboard 5.3 cycles per issue"},
-                 ("batch", "exact"): {"issue_active_pct": 71.6, "lanes_per_warp_instruction": 14.10,
-                                      "fp64_pipe_active_pct": 24.8, "fma_pipe_active_pct": 16.9, "l1_hit_pct": 84.8,
-                                      "l2_hit_pct": 88.5, "top_stall": "wait 2.9 cycles per issue"},
-                 ("batch", "fast"): {"issue_active_pct": 75.4, "lanes_per_warp_instruction": 14.36,
-                                     "fp64_pipe_active_pct": 26.1, "fma_pipe_active_pct": 16.6, "l1_hit_pct": 81.3,
-                                     "l2_hit_pct": 88.6, "top_stall": "wait 2.9 cycles per issue"}}
+NCU_EXECUTION = {("triangle_heavy", "exact"): {"issue_active_pct": 58.8, "lanes_per_warp_instruction": 7.45,
+                                               "fp64_pipe_active_pct": 27.1, "fma_pipe_active_pct": 10.4,
+                                               "l1_hit_pct": 77.8, "l2_hit_pct": 84.6,
+                                               "top_stall": "long_scoreboard 5.1 cycles per issue"},
+                 ("triangle_heavy", "fast"): {"issue_active_pct": 59.4, "lanes_per_warp_instruction": 7.47,
+                                              "fp64_pipe_active_pct": 27.6, "fma_pipe_active_pct": 10.5,
+                                              "l1_hit_pct": 78.7, "l2_hit_pct": 84.5,
+                                              "top_stall": "long_scoreboard 5.5 cycles per issue"},
+                 ("batch", "exact"): {"issue_active_pct": 71.6, "lanes_per_warp_instruction": 14.12,
+                                      "fp64_pipe_active_pct": 26.5, "fma_pipe_active_pct": 17.2,
+                                      "l1_hit_pct": 87.3, "l2_hit_pct": 88.3,
+                                      "top_stall": "wait 3.0 cycles per issue"},
+                 ("batch", "fast"): {"issue_active_pct": 74.5, "lanes_per_warp_instruction": 14.34,
+                                     "fp64_pipe_active_pct": 26.7, "fma_pipe_active_pct": 17.1,
+                                     "l1_hit_pct": 82.8, "l2_hit_pct": 88.2,
+                                     "top_stall": "wait 3.0 cycles per issue"}}
 # The batched launch, captured whole (rank 0's batch, one launch), by precision.
-NCU_DRAM_BYTES_BATCH = {"exact": 0.095720e9 + 0.987772e9, "fast": 0.129497e9 + 1.905857e9}
+NCU_DRAM_BYTES_BATCH = {"exact": 0.091824e9 + 0.763702e9, "fast": 0.129599e9 + 1.644152e9}
 
 
 FP32_LANES_PER_SM = 128
