@@ -51,6 +51,13 @@ static void parallel_ranges(size_t n, size_t grain, const F& f) {
   for (size_t i = 0; i < started; ++i) team[i].join();
 }
 
+void touch_pages(void* p, size_t bytes) {
+  constexpr size_t page = 4096;
+  parallel_ranges(bytes / page, 4096, [&](size_t begin, size_t end) {
+    for (size_t i = begin; i < end; ++i) static_cast<volatile char*>(p)[i * page] = 0;
+  });
+}
+
 /* ------------------------------------------------------------ AABB ---- */
 /* src/aabb.zig */
 struct Box {

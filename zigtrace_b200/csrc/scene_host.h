@@ -143,6 +143,9 @@ DCamera camera_init(const zt_camera_config& cfg, double aspect);
  * (flatten_on_device, bvh_build.cu) and sets the view's root and the float
  * records' root and margins (fast_eps) as far as the root box decides them. */
 void flatten_scene(const zt_scene* s, FlatScene* out, bool with_tree = true);
+/* Writes to every page of [p, p + bytes), from several threads where it is
+ * large. */
+void touch_pages(void* p, size_t bytes);
 /* Shapes, permutation and nodes of a scene in device memory. */
 struct DeviceTree {
   const zt_shape* shapes;
