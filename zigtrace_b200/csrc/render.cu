@@ -526,8 +526,8 @@ constexpr int kMegaThreadsPerSmNoNee = 896;
  * float-walk instances measured fastest at 1024 (64 registers): 1M-triangle
  * terrain (16 spp) 31.1 ms against 31.2 at 896, 33.4 at 768 and 31.7 at
  * 1152; the sphere-field batch 51.7 against 51.6, 52.7 and 57.0.  The
- * checked walk without light sampling is built for 896: random spheres 3.98
- * against 4.07 ms. */
+ * checked walk without light sampling is built for 896: random spheres 3.82
+ * against 4.18 ms, the batch 51.9 against 53.6. */
 __host__ __device__ constexpr int mega_threads_per_sm(bool nee, int walk) {
   return walk == kWalkF64 ? (nee ? kMegaThreadsPerSm : kMegaThreadsPerSmNoNee)
                           : (walk == kWalkFloatChecked && !nee ? 896 : 1024);

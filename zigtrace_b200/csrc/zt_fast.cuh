@@ -99,8 +99,8 @@
  * 3.87 and 5.6.  The f64 comparisons also take less time than the conversions
  * did (random spheres 3.78 -> 3.61 ms, terrain unchanged).
  * Measured, against the f64 walk with its 128-byte records: 250k-triangle
- * terrain 961x541x16 14.56 -> 11.14 ms, random spheres 1280x720x16 5.35 ->
- * 4.09 ms, 256 sphere fields 71.9 -> 54.8 ms.
+ * terrain 961x541x16 15.0 -> 11.2 ms, random spheres 1280x720x16 5.34 ->
+ * 3.75 ms, 256 sphere fields 71.9 -> 51.9 ms.
  *
  * Stack entries are 8 bytes (packed payload word + float entry distance),
  * 4 bytes in the any-hit walk.
